@@ -57,6 +57,7 @@
 //          blocks I = 0..DP/8-1 then their lo parts; LBO = 128, SBO = 256,
 //          N = 2 DP.
 #include "common.cuh"
+#include "sweep.cuh"
 
 namespace lakde {
 namespace tc {
@@ -1110,19 +1111,6 @@ __global__ void __launch_bounds__(NTHR_ALL, 1) tc_kernel(Args g) {
   if (warp == 0) tmem_dealloc(tmem, 2 * K::ACC_COLS);
 }
 
-// out[q] = -log N + logsumexp over the chunks' (max, sum) partials
-__global__ void pred_fold_kernel(const float *__restrict__ ws_m, const float *__restrict__ ws_s,
-                                 float *__restrict__ out, int64_t Nq, int64_t nchunks, float log_n) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= Nq) return;
-  float M = -INFINITY;
-  for (int64_t c = 0; c < nchunks; ++c) M = fmaxf(M, ws_m[c * Nq + q]);
-  float S = 0.f;
-  if (M != -INFINITY)
-    for (int64_t c = 0; c < nchunks; ++c) S += ws_s[c * Nq + q] * expf(ws_m[c * Nq + q] - M);
-  out[q] = (M == -INFINITY) ? M : (M + logf(S)) - log_n;
-}
-
 // W_triu (dense, upper) -> W cores: element X[i][j] = W_triu[j][i] (i >= j) of
 // segment J = j / 8, row block I = i / 8, core (j % 8) / 4, row i % 8, column
 // j % 4, its tf32 hi part in the segment's hi run and lo = tf32(x - hi) in the
@@ -1488,7 +1476,7 @@ extern "C" int lakde_log_pred_density_tc(int dtype, int64_t N, int64_t Nq, int64
     return (int)LAKDE_OK;
   });
   if (st) return st;
-  tc::pred_fold_kernel<<<(unsigned)((Nq + 255) / 256), 256, 0, as_stream(stream)>>>(
+  sweep::fold_kernel<float><<<(unsigned)((Nq + 31) / 32), 256, 0, as_stream(stream)>>>(
       g.ws_m, g.ws_s, static_cast<float *>(out), Nq, grid, (float)log((double)N));
   return check_launch("log_pred_density_tc_fold");
 }
