@@ -13,116 +13,156 @@
 // S_c[n] = sum_y c_ny d d^T, from which the host finishes d/dL_n with D x D
 // products (sum_y c_ny z z^T = W_triu^T S_c W_triu).
 #include "common.cuh"
+#include "sweep.cuh"
 
 namespace lakde {
 
+// The staged factor in the unrolled layout at every DP (the pass needs all of
+// z at once); two queries a thread up to 32 dimensions in float32 (z and the
+// score take 2 DP registers a query), else one.  A query's coordinates are
+// read once per kernel, from a shared-memory column of the thread.
 template <typename T, int DP>
-struct BwdCfg {
-  static constexpr int QT = 128;
-  static constexpr int KT = DP <= 16 ? 16 : (DP <= 32 ? 8 : 4);
-  static constexpr int TS = Tri<T>::size(DP);
-  // packed factor, centre, log coefficient, h
-  static constexpr int per_kernel = ((TS + DP + 2 + Tri<T>::V - 1) / Tri<T>::V) * Tri<T>::V;
-  static constexpr size_t smem = (size_t)KT * per_kernel * sizeof(T) + (size_t)KT * 4 * sizeof(T);
+struct BwdCfg : sweep::Cfg<T, DP, false> {
+  using L = sweep::Cfg<T, DP, false>;
+  static constexpr int P = sizeof(T) == 4 && DP <= 32 ? 2 : 1;
+  static constexpr int TILE = sweep::THREADS * P;
+  static constexpr int KT = DP <= 8 ? 16 : DP <= 32 ? 8 : 2;
+  static constexpr int OCC = DP <= 32 && sizeof(T) == 4 ? 3 : 2;
+  // two stages, the queries, the warps' sums of g w
+  static constexpr size_t smem =
+      (2 * (size_t)KT * L::KS + (size_t)DP * TILE + (size_t)KT * (sweep::THREADS / 32)) * sizeof(T);
 };
 
-static int64_t bwd_chunk(int64_t N, int64_t Nq, int kt) {
-  const int64_t q_tiles = (Nq + 127) / 128;
-  const int64_t target = 148 * 4;
-  int64_t nchunks = (target + q_tiles - 1) / q_tiles;
+// Chunks of kernels: three waves of the resident CTAs with the query tiles.
+template <typename T, int DP>
+static int64_t bwd_chunk(int64_t N, int64_t Nq) {
+  using C = BwdCfg<T, DP>;
+  const int64_t tiles = (Nq + C::TILE - 1) / C::TILE;
+  int64_t nchunks = (int64_t)148 * 3 * C::OCC / tiles;
   if (nchunks < 1) nchunks = 1;
-  int64_t chunk = (N + nchunks - 1) / nchunks;
-  chunk = ((chunk + kt - 1) / kt) * kt;
-  return chunk < kt ? kt : chunk;
+  const int64_t chunk = (N + nchunks - 1) / nchunks;
+  return chunk < 4 ? 4 : chunk;
 }
 
-// (U z)_i = sum_{j >= i} U[i][j] z_j for the packed upper factor (column j holds rows 0..j)
+// Bound by the FMA pipe and the broadcast reads of U (twice per kernel: z =
+// U^T d, then U z), with the accurate log1p / exp and one division a pair.
+// 20,000 kernels x 4,096 queries at d = 21, float32: 10.2 -> 2.7 ms against one
+// query per thread with element-wise reads of U in the second product.
 template <typename T, int DP>
-__device__ __forceinline__ void upper_times(const T *__restrict__ sU, const T (&z)[DP], T (&out)[DP]) {
-#pragma unroll
-  for (int i = 0; i < DP; ++i) out[i] = T(0);
-  int off = 0;
-#pragma unroll
-  for (int j = 0; j < DP; ++j) {
-#pragma unroll
-    for (int i = 0; i <= j; ++i) out[i] = fma(sU[off + i], z[j], out[i]);
-    off += Tri<T>::col_len(j);
-  }
-}
-
-template <typename T, int DP>
-__global__ void __launch_bounds__(128) pred_bwd_pairs_kernel(
+__global__ void __launch_bounds__(sweep::THREADS, BwdCfg<T, DP>::OCC) pred_bwd_pairs_kernel(
     const T *__restrict__ X, const T *__restrict__ W, const T *__restrict__ nu, const T *__restrict__ lcoef,
     const T *__restrict__ Y, const T *__restrict__ outp, const T *__restrict__ gout, T *__restrict__ cw,
     T *__restrict__ sw_part, T *__restrict__ score_part, int64_t N, int64_t Nq, int D, int64_t chunk, int64_t q_tiles,
     T log_n) {
   using C = BwdCfg<T, DP>;
+  using L = typename C::L;
+  constexpr int P = C::P, V = L::V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sbase = reinterpret_cast<T *>(smem_raw);
-  T *sred = sbase + C::KT * C::per_kernel;  // [KT][4] warp partials of sum_y g w
+  T *st = reinterpret_cast<T *>(smem_raw);
+  T *ys = st + 2 * C::KT * L::KS;
+  T *sred = ys + DP * C::TILE;  // [KT][4] warp sums of g w
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t qt = blockIdx.x % q_tiles;
   const int64_t ch = blockIdx.x / q_tiles;
-  const int64_t q = qt * C::QT + tid;
-  const bool qv = q < Nq;
   const int64_t n_begin = ch * chunk;
   const int64_t n_end = (n_begin + chunk < N) ? n_begin + chunk : N;
-
-  T y[DP];
-#pragma unroll
-  for (int d = 0; d < DP; ++d) y[d] = (qv && d < D) ? Y[q * D + d] : T(0);
-  const T ly = qv ? outp[q] + log_n : T(0);
-  const T g = qv ? gout[q] : T(0);
-  T score[DP];
-#pragma unroll
-  for (int d = 0; d < DP; ++d) score[d] = T(0);
-
-  for (int64_t n0 = n_begin; n0 < n_end; n0 += C::KT) {
-    const int cnt = (int)((n_end - n0) < C::KT ? (n_end - n0) : C::KT);
-    __syncthreads();
-    for (int k = 0; k < cnt; ++k) {
-      T *sk = sbase + k * C::per_kernel;
-      const int64_t n = n0 + k;
-      load_tri<T, DP>(sk, W + n * (int64_t)D * D, D, 1, D, true, tid, C::QT);
-      for (int d = tid; d < DP; d += C::QT) sk[C::TS + d] = d < D ? X[n * D + d] : T(0);
-      if (tid == 0) {
-        sk[C::TS + DP] = lcoef[n];
-        sk[C::TS + DP + 1] = (nu[n] + T(1)) / T(2);
-      }
+  auto count = [&](int64_t n0) { return (int)((n_end - n0) < C::KT ? (n_end - n0) : C::KT); };
+  auto stage = [&](int s, int64_t n0) {
+    T *d = st + s * C::KT * L::KS;
+    const int cnt = count(n0);
+    sweep::stage_kernels<T, DP, L>(d, W, (int64_t)D * D, D, 1, X, D, 1, n0, cnt, D, tid);
+    for (int k = tid; k < cnt; k += sweep::THREADS) {
+      sweep::cp_async_elem(d + k * L::KS + L::S0, lcoef + n0 + k);
+      sweep::cp_async_elem(d + k * L::KS + L::S0 + 1, nu + n0 + k);
     }
+  };
+  for (int e = tid; e < 2 * C::KT * L::KS; e += sweep::THREADS) st[e] = T(0);
+  __syncthreads();
+  stage(0, n_begin);
+  sweep::cp_async_commit();
+
+  T ly[P], g[P], score[P][DP];
+  T *col = ys + tid * P;
+#pragma unroll
+  for (int p = 0; p < P; ++p) {
+    const int64_t q = qt * C::TILE + tid + (int64_t)p * sweep::THREADS;
+    const bool qv = q < Nq;
+    ly[p] = qv ? outp[q] + log_n : T(0);
+    g[p] = qv ? gout[q] : T(0);
+#pragma unroll
+    for (int d = 0; d < DP; ++d) {
+      col[d * C::TILE + p] = (qv && d < D) ? Y[q * D + d] : T(0);
+      score[p][d] = T(0);
+    }
+  }
+
+  int b = 0;
+  for (int64_t n0 = n_begin; n0 < n_end; n0 += C::KT, b ^= 1) {
+    if (n0 + C::KT < n_end) stage(b ^ 1, n0 + C::KT);
+    sweep::cp_async_commit();
+    sweep::cp_async_wait<1>();
     __syncthreads();
+    const int cnt = count(n0);
     for (int k = 0; k < cnt; ++k) {
-      const T *sk = sbase + k * C::per_kernel;
-      const int64_t n = n0 + k;
-      T delta[DP], z[DP];
+      const T *sk = st + (b * C::KT + k) * L::KS;
+      sweep::Pair<T> acc[P][(DP + 1) / 2];
+      sweep::products<L, T, DP, P>(sk, [&](int p, int j) { return col[j * C::TILE + p]; }, acc);
+      T q[P], f[P];
+      sweep::squares<T, DP, P>(acc, q);
+      const T lc = sk[L::S0], h = (sk[L::S0 + 1] + T(1)) / T(2);
+      T gw = T(0);
 #pragma unroll
-      for (int d = 0; d < DP; ++d) delta[d] = y[d] - sk[C::TS + d];
-      const T Q = quad_tri_z<T, DP>(sk, delta, z);
-      const T h = sk[C::TS + DP + 1];
-      const T lp = sk[C::TS + DP] - h * log1p(Q);
-      const T w = qv ? exp(lp - ly) : T(0);
-      const T c = g * w / (T(1) + Q);
-      if (qv) cw[n * Nq + q] = c;
-      // score: g w (-2 h / (1 + Q)) U z = -2 h c U z
-      T uz[DP];
-      upper_times<T, DP>(sk, z, uz);
-      const T f = T(-2) * h * c;
+      for (int p = 0; p < P; ++p) {
+        const int64_t m = qt * C::TILE + tid + (int64_t)p * sweep::THREADS;
+        const T lp = lc - h * log1p(q[p]);
+        const T w = m < Nq ? exp(lp - ly[p]) : T(0);
+        const T c = g[p] * w / (T(1) + q[p]);
+        if (m < Nq) cw[(n0 + k) * Nq + m] = c;
+        f[p] = T(-2) * h * c;
+        gw += g[p] * w;
+      }
+      // score: g w (-2 h / (1 + Q)) U z = -2 h c U z, row j of U against z
 #pragma unroll
-      for (int d = 0; d < DP; ++d) score[d] = fma(f, uz[d], score[d]);
+      for (int j = 0; j < DP; ++j) {
+        // the loads of two rows at a time (hoisting more of them spills)
+        if ((j & 1) == 0) asm volatile("" ::: "memory");
+        T uz[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) uz[p] = T(0);
+#pragma unroll
+        for (int i0 = V * (j / V); i0 < L::DPV; i0 += V) {
+          T u[V];
+          sweep::load_vec<T>(sk + L::at(j, i0), u);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const int i = i0 + v;
+            if (i < j || i >= DP) continue;
+#pragma unroll
+            for (int p = 0; p < P; ++p) uz[p] = fma(u[v], (i & 1) ? acc[p][i / 2].hi() : acc[p][i / 2].lo(), uz[p]);
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) score[p][j] = fma(f[p], uz[p], score[p][j]);
+      }
       // sum over this CTA's queries of g w for kernel n
-      const T gw = warp_sum(g * w);
+      gw = warp_sum(gw);
       if (lane == 0) sred[k * 4 + warp] = gw;
     }
-    __syncthreads();
-    for (int k = tid; k < cnt; k += C::QT) {
+    __syncthreads();  // the sums are written, the stage is free to refill
+    for (int k = tid; k < cnt; k += sweep::THREADS) {
       const T s = sred[k * 4 + 0] + sred[k * 4 + 1] + sred[k * 4 + 2] + sred[k * 4 + 3];
       sw_part[qt * N + n0 + k] = s;
     }
+    // (the next group's sums are written after its own barrier above)
   }
-  if (qv) {
 #pragma unroll
-    for (int d = 0; d < DP; ++d)
-      if (d < D) score_part[(ch * Nq + q) * D + d] = score[d];
+  for (int p = 0; p < P; ++p) {
+    const int64_t q = qt * C::TILE + tid + (int64_t)p * sweep::THREADS;
+    if (q < Nq) {
+#pragma unroll
+      for (int d = 0; d < DP; ++d)
+        if (d < D) score_part[(ch * Nq + q) * D + d] = score[p][d];
+    }
   }
 }
 
@@ -135,60 +175,71 @@ __global__ void sum_parts_kernel(const T *__restrict__ parts, T *__restrict__ ou
   out[i] = s;
 }
 
-// S_c[n] = sum_y c[n, y] (y - x_n)(y - x_n)^T over all queries; one CTA per
-// kernel, threads own 4x4 blocks of the lower triangle, queries staged 64 at a
-// time as centred differences.
+// S_c[n] = sum_y c[n, y] (y - x_n)(y - x_n)^T over all queries.  A thread owns
+// a 4 x 4 block of one kernel's lower triangle; a CTA takes G kernels packed
+// densely into its threads and stages the raw queries 64 at a time for all of
+// them (centred in registers), so the staging and its barriers are paid once
+// per G kernels and the lanes are full.  One kernel per CTA left 11 of 32 lanes
+// idle at 24 dimensions and waited on its own staging: 7.7 ms for 20,000
+// kernels x 4,096 queries at d = 21, now 2.6 ms (issue 70 %).
 template <typename T, int DP>
 struct DenseScatterCfg {
   static constexpr int NB = DP < 4 ? 1 : DP / 4;
   static constexpr int NBLK = NB * (NB + 1) / 2;
-  static constexpr int THREADS = ((NBLK + 31) / 32) * 32;
+  static constexpr int GMAX = NBLK >= 128 ? 2 : 256 / NBLK > 32 ? 32 : 256 / NBLK;  // kernels per CTA
   static constexpr int CH = 64;
   static constexpr int LD = (DP < 4 ? 4 : DP) + 4;
 };
 
 template <typename T, int DP>
-__global__ void dense_scatter_kernel(const T *__restrict__ cw, const T *__restrict__ X, const T *__restrict__ Y,
-                                     T *__restrict__ S, int64_t N, int64_t Nq, int D) {
+__global__ void __launch_bounds__(320) dense_scatter_kernel(const T *__restrict__ cw, const T *__restrict__ X,
+                                                            const T *__restrict__ Y, T *__restrict__ S, int64_t N,
+                                                            int64_t Nq, int D, int G) {
   using C = DenseScatterCfg<T, DP>;
+  constexpr int V = 16 / (int)sizeof(T);
   __shared__ __align__(16) T sd[C::CH][C::LD];
-  __shared__ T sv[C::CH];
-  __shared__ T sxn[C::LD];
-  const int64_t n = blockIdx.x;
-  const int tid = threadIdx.x;
-  int bi = -1, bj = -1;
-  {
-    int e = 0;
-    for (int i = 0; i < C::NB; ++i)
-      for (int j = 0; j <= i; ++j, ++e)
-        if (e == tid) {
-          bi = i;
-          bj = j;
-        }
-  }
-  for (int d = tid; d < C::LD; d += blockDim.x) sxn[d] = d < D ? X[n * D + d] : T(0);
-  T acc[4][4];
+  __shared__ T sv[C::GMAX][C::CH];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int64_t n0 = (int64_t)blockIdx.x * G;
+  const int g = tid / C::NBLK, e = tid % C::NBLK;
+  const int64_t n = n0 + g;
+  const bool own = g < G && n < N;
+  int bi = 0;
+  while ((bi + 1) * (bi + 2) / 2 <= e) ++bi;
+  const int bj = e - bi * (bi + 1) / 2;
+  T xa[4], xb[4], acc[4][4];
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < 4; ++p) {
+    xa[p] = (own && 4 * bi + p < D) ? X[n * D + 4 * bi + p] : T(0);
+    xb[p] = (own && 4 * bj + p < D) ? X[n * D + 4 * bj + p] : T(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[p][q] = T(0);
+  }
   for (int64_t base = 0; base < Nq; base += C::CH) {
     const int cnt = (int)((Nq - base) < C::CH ? (Nq - base) : C::CH);
     __syncthreads();
-    for (int e = tid; e < C::CH * C::LD; e += blockDim.x) {
-      const int pp = e / C::LD, d = e % C::LD;
-      sd[pp][d] = (pp < cnt && d < D) ? Y[(base + pp) * D + d] - sxn[d] : T(0);
+    for (int pp = tid >> 5; pp < cnt; pp += blockDim.x >> 5)
+      for (int d = lane; d < C::LD; d += 32) sd[pp][d] = d < D ? Y[(base + pp) * D + d] : T(0);
+    for (int f = tid; f < G * C::CH; f += blockDim.x) {
+      const int k = f / C::CH, pp = f % C::CH;
+      sv[k][pp] = (n0 + k < N && pp < cnt) ? cw[(n0 + k) * Nq + base + pp] : T(0);
     }
-    for (int pp = tid; pp < C::CH; pp += blockDim.x) sv[pp] = pp < cnt ? cw[n * Nq + base + pp] : T(0);
     __syncthreads();
-    if (bi >= 0) {
+    if (own) {
+#pragma unroll 2
       for (int pp = 0; pp < cnt; ++pp) {
-        const T v = sv[pp];
+        const T v = sv[g][pp];
         T a[4], b[4];
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          a[p] = sd[pp][4 * bi + p];
-          b[p] = v * sd[pp][4 * bj + p];
+        for (int p = 0; p < 4; p += V) {
+          T u[V], w[V];
+          sweep::load_vec<T>(&sd[pp][4 * bi + p], u);
+          sweep::load_vec<T>(&sd[pp][4 * bj + p], w);
+#pragma unroll
+          for (int k = 0; k < V; ++k) {
+            a[p + k] = u[k] - xa[p + k];
+            b[p + k] = v * (w[k] - xb[p + k]);
+          }
         }
 #pragma unroll
         for (int p = 0; p < 4; ++p)
@@ -197,7 +248,7 @@ __global__ void dense_scatter_kernel(const T *__restrict__ cw, const T *__restri
       }
     }
   }
-  if (bi < 0) return;
+  if (!own) return;
   T *o = S + n * (int64_t)D * D;
 #pragma unroll
   for (int p = 0; p < 4; ++p)
@@ -210,29 +261,25 @@ __global__ void dense_scatter_kernel(const T *__restrict__ cw, const T *__restri
     }
 }
 
-static int bwd_kt(int dtype, int64_t D) {
-  int kt = 0;
-  dispatch_float(dtype, [&](auto t0) {
-    using T = decltype(t0);
-    return dispatch_dp(D, [&](auto dp) {
-      kt = BwdCfg<T, decltype(dp)::value>::KT;
-      return 0;
-    });
-  });
-  return kt;
-}
-
 }  // namespace lakde
 
 using namespace lakde;
 
 extern "C" size_t lakde_log_pred_density_bwd_workspace(int dtype, int64_t N, int64_t Nq, int64_t D) {
   if (N <= 0 || Nq <= 0 || D < 1 || D > kMaxDim || (dtype != LAKDE_F32 && dtype != LAKDE_F64)) return 0;
-  const int64_t chunk = bwd_chunk(N, Nq, bwd_kt(dtype, D));
-  const int64_t nchunks = (N + chunk - 1) / chunk;
-  const int64_t q_tiles = (Nq + 127) / 128;
-  const size_t es = dtype == LAKDE_F32 ? 4 : 8;
-  return (size_t)(q_tiles * N + nchunks * Nq * D) * es;
+  size_t bytes = 0;
+  dispatch_float(dtype, [&](auto t0) {
+    using T = decltype(t0);
+    return dispatch_dp(D, [&](auto dp) {
+      using C = BwdCfg<T, decltype(dp)::value>;
+      const int64_t chunk = bwd_chunk<T, decltype(dp)::value>(N, Nq);
+      const int64_t nchunks = (N + chunk - 1) / chunk;
+      const int64_t q_tiles = (Nq + C::TILE - 1) / C::TILE;
+      bytes = (size_t)(q_tiles * N + nchunks * Nq * D) * sizeof(T);
+      return 0;
+    });
+  });
+  return bytes;
 }
 
 extern "C" int lakde_log_pred_density_bwd(int dtype, int64_t N, int64_t Nq, int64_t D, const void *X,
@@ -265,9 +312,9 @@ extern "C" int lakde_log_pred_density_bwd(int dtype, int64_t N, int64_t Nq, int6
     return dispatch_dp(D, [&](auto dp) {
       constexpr int DP = decltype(dp)::value;
       using C = BwdCfg<T, DP>;
-      const int64_t chunk = bwd_chunk(N, Nq, C::KT);
+      const int64_t chunk = bwd_chunk<T, DP>(N, Nq);
       const int64_t nchunks = (N + chunk - 1) / chunk;
-      const int64_t q_tiles = (Nq + C::QT - 1) / C::QT;
+      const int64_t q_tiles = (Nq + C::TILE - 1) / C::TILE;
       T *sw_part = static_cast<T *>(workspace);
       T *score_part = sw_part + q_tiles * N;
       auto kern = pred_bwd_pairs_kernel<T, DP>;
@@ -278,7 +325,7 @@ extern "C" int lakde_log_pred_density_bwd(int dtype, int64_t N, int64_t Nq, int6
           return (int)LAKDE_ECUDA;
         }
       }
-      kern<<<(unsigned)(q_tiles * nchunks), C::QT, C::smem, as_stream(stream)>>>(
+      kern<<<(unsigned)(q_tiles * nchunks), sweep::THREADS, C::smem, as_stream(stream)>>>(
           static_cast<const T *>(X), static_cast<const T *>(W_triu), static_cast<const T *>(nu),
           static_cast<const T *>(log_coeff), static_cast<const T *>(Y), static_cast<const T *>(out),
           static_cast<const T *>(grad_out), static_cast<T *>(cw), sw_part, score_part, N, Nq, (int)D, chunk, q_tiles,
@@ -291,9 +338,13 @@ extern "C" int lakde_log_pred_density_bwd(int dtype, int64_t N, int64_t Nq, int6
           score_part, static_cast<T *>(grad_Y), Nq * D, nchunks);
       if (int st = check_launch("log_pred_density_bwd_score")) return st;
       using SC = DenseScatterCfg<T, DP>;
-      dense_scatter_kernel<T, DP><<<(unsigned)N, SC::THREADS, 0, as_stream(stream)>>>(
+      // as many kernels per CTA as fit, but at least about four CTAs an SM
+      int64_t G = N / (148 * 4);
+      G = G < 1 ? 1 : G > SC::GMAX ? SC::GMAX : G;
+      const unsigned threads = (unsigned)((G * SC::NBLK + 31) / 32) * 32;
+      dense_scatter_kernel<T, DP><<<(unsigned)((N + G - 1) / G), threads, 0, as_stream(stream)>>>(
           static_cast<const T *>(cw), static_cast<const T *>(X), static_cast<const T *>(Y), static_cast<T *>(S_c), N,
-          Nq, (int)D);
+          Nq, (int)D, (int)G);
       return check_launch("log_pred_density_bwd_scatter");
     });
   });
