@@ -181,10 +181,24 @@ __device__ __forceinline__ double digamma_d(double x) {
   return acc + log(x) - 0.5 / x - series;
 }
 
-// sum_{i=1..D} psi(a + (1 - i)/2)
+// sum_{i=1..D} psi(a + (1 - i)/2), NaN when an argument is not positive.  The
+// arguments form two chains of unit steps, a, a - 1, .. and h, h - 1, .. with
+// h = a - 1/2, and psi(x - 1) = psi(x) - 1 / (x - 1), so
+//   sum_{j < n} psi(x - j) = n psi(x) - sum_{k=1..n-1} (n - k) / (x - k):
+// two series and one division per step of both chains, instead of a series,
+// a logarithm and up to six recurrence divisions per term (at D = 63 the
+// E-step's row constants took 25k cycles per 32 rows of its metadata warp).
 __device__ __forceinline__ double mvdigamma_d(double a, int D) {
-  double s = 0.0;
-  for (int i = 1; i <= D; ++i) s += digamma_d(a + 0.5 * (1 - i));
+  if (!(a + 0.5 * (1 - D) > 0.0)) return nan("");
+  const int n1 = (D + 1) / 2, n2 = D / 2;
+  const double h = a - 0.5;
+  double s = n1 * digamma_d(a);
+  if (n2 > 0) s += n2 * digamma_d(h);
+  for (int k = 1; k < n2; ++k) {
+    const double x = a - k, y = h - k;
+    s -= ((n1 - k) * y + (n2 - k) * x) / (x * y);
+  }
+  if (n2 > 0 && n1 > n2) s -= 1.0 / (a - n2);  // odd D: the first chain is one longer
   return s;
 }
 

@@ -389,8 +389,7 @@ struct Kern {
         // 0.5 (psi_D(nu / 2) + D log 2 + logdet W), -nu / 2
         const float nv = g.nu[n];
         const float ld = g.logdet[n];
-        double md = 0.0;
-        for (int i = 1; i <= g.D; ++i) md += digamma_d(0.5 * (double)nv + 0.5 * (1 - i));
+        const double md = mvdigamma_d(0.5 * (double)nv, g.D);
         c0 = (float)(0.5 * (md + g.D * 0.69314718055994530942 + (double)ld));
         c1 = -0.5f * nv;
       } else if (MODE == PRED) {
