@@ -18,33 +18,53 @@
 // (D_hi + D_lo) (W_hi + W_lo) (two MMAs per K step against [W_hi | W_lo]);
 // what remains is the rounding of lo, below 2^-22 relative with random sign.
 //
-// One persistent CTA per SM, 384 threads in four roles, pipelined over
-// 128-pair tiles with mbarriers:
-//   * a metadata warp takes kernel rows 32 at a time (an atomic row queue
-//     over the caller's longest-first order, or a static stride), one lane
-//     per row for the dependent loads and the E-step's digamma sums, and
-//     writes each tile's row, pair range, column indices and weights into a
-//     ring of 8 slots, loading the next tile's indices while it writes one;
-//   * two gather warps copy each tile's pair rows (rows of X padded to a
-//     multiple of 16 bytes) into one of two raw stages with cp.async, the
-//     first also its kernel centre and, for the first tile of a row, the row's
-//     W cores into one of two B stages by bulk copy, after the stage's last
-//     MMAs committed;
-//   * 8 consumer warps convert tile t (centre, M-step: scale by sqrt r, split
-//     into the hi / lo core-matrix tile) and read the previous tile's
-//     accumulator (one TMEM lane per pair) to write log rho / S_n / the
-//     running log-sum-exp;
+// Persistent CTAs of warps in four roles, pipelined over 128-pair tiles with
+// mbarriers (one CTA an SM at 48 and 64 padded dimensions, two below,
+// where a tile's work is too short for one CTA to cover its own latencies):
+//   * converter warps hold the next tile's pair rows in registers: 16-byte
+//     loads, the lanes of a row side by side so that a warp instruction reads
+//     whole lines.  They centre, (M-step: scale by sqrt r,) split and store tile
+//     t into the hi / lo core-matrix tile;
+//   * epilogue warpgroups take turns over the tiles (M-step: rows): read the
+//     accumulator (one TMEM lane per pair) and write log rho / S_n / the running
+//     log-sum-exp;
+//   * a planner warp takes kernel rows up to 32 at a time (an atomic row queue
+//     over the caller's longest-first order, or a static stride), one lane per
+//     row for the dependent loads and the E-step's digamma sums, and plans 32
+//     tiles at once, one per lane, into a ring of 64 (row, pair range, row
+//     constants);
+//   * two index warps validate the tiles' column indices and write them (M-step:
+//     with sqrt r) into a ring of 8 slots;
+//   * two copy warps bring a row's W cores into one of two B stages, after the
+//     stage's last MMAs committed;
 //   * an MMA warp issues each converted tile's MMAs into one of two TMEM
 //     accumulators and commits them to mbarriers.
-// Every wait is bounded: on a time-out the kernel sets *err, waits (bounded)
-// for its own copies and MMAs in flight, frees its TMEM and returns.
+// The predictive density keeps its CTA's 256 queries in registers for the whole
+// launch (two tiles per kernel) and its running (max, sum) pairs too.
+// Every wait is bounded: on a time-out the warp sets *err, waits (bounded) for
+// its own copies and MMAs in flight, and the CTA frees its TMEM and returns.
+// No warp waits on a named barrier, which could not time out.
+//
+// What bounds it: a full E-step tile at DP = 64 moves about 220 KB through
+// shared memory (128 KB of operands of its 16 MMAs, 64 KB stored by the
+// converters, 18 KB of W cores, the barriers) at 128 bytes a cycle, so 1.7k of the
+// 2.3k to 3.2k cycles it takes; the MMAs alone are 1.0k.  What it replaced: two
+// gather warps copied the rows into shared memory with 16-byte cp.async, 64
+// bytes of a line per row and instruction (2.5k cycles a tile), eight warps read
+// them back to convert, met at a named barrier per tile and all ran the
+// epilogue, and one warp planned tile by tile.  Measured, 50,000 rows, before ->
+// now, E-step: d = 63, 100 pairs a row 0.95 -> 0.55 ms, 30 pairs 0.87 -> 0.49;
+// d = 21, 64 pairs 0.54 -> 0.28; d = 13, 40 pairs 0.46 -> 0.19.  M-step: d = 63 0.91
+// -> 0.61 and 0.80 -> 0.46 ms, d = 21 0.69 -> 0.31, d = 13 0.67 -> 0.23.  Predictive
+// density, 5,000 kernels x 4,096 queries: d = 63 2.12 -> 1.24 ms, d = 43 1.76 -> 1.18,
+// d = 21 1.39 -> 0.68, d = 13 1.39 -> 0.48.
 //
 // Shared-memory operand layout (canonical, no swizzle; a core matrix is 8 rows
 // x 16 bytes = 8 x 4 tf32):
-//   tile   E-step / predictive density: 16 pair groups x 32 cores: core
-//          c < 16 holds dims 4c..4c+3 of the 8 pairs' hi parts, core 16 + c
-//          the lo parts; the A operand (K-major, M = pairs): LBO = 128 (next
-//          4 dims), SBO = 4096 (next 8 pairs).
+//   tile   E-step / predictive density (K-major, M = pairs): the 8 pairs of a
+//          group, their DP / 4 hi cores then as many lo cores, LBO = 144 apart
+//          (next 4 dims; 144 rather than 128 puts the lanes of a row on
+//          distinct bank groups), SBO = 2 (DP / 4) 144 (next 8 pairs).
 //          M-step: G^T, rows = [hi dims 0..63; lo dims 0..63], K = pairs:
 //          core (row group r / 8, pair quad p / 4) at (r / 8) GT_SBO +
 //          (p / 4) 128; A = [G_hi; G_lo]^T (M = 128) and B = G_hi (its first
@@ -63,14 +83,15 @@ namespace lakde {
 namespace tc {
 
 constexpr int MT = 128;        // pairs (queries) per tile: the MMA M
-constexpr int NTHR = 256;      // 8 consumer warps (two more produce)
-constexpr int NS = 8;          // metadata slots
-constexpr int NGW = 2;         // gather warps (four measured no faster: the scattered copies, not their issue, set the rate)
-constexpr int RAW_STRIDE = 272;  // bytes per staged pair row: 64 floats + 16 bytes against bank conflicts
+constexpr int NCOPY = 2;       // copy warps
+constexpr int NIDX = 2;        // index warps
+constexpr int NPL = 64;        // planned tiles: two halves of 32
+constexpr int NS = 8;          // index slots
 constexpr uint32_t kSpinLimit = 1u << 26;
 constexpr uint64_t kWaitLimitNs = 1500000000ull;  // 1.5 s: far above any copy or MMA of one tile
-constexpr int PQ = 2048;       // queries per predictive-density launch
+constexpr int QB = 2 * MT;     // queries per predictive-density CTA
 constexpr uint32_t GT_SBO = 4112;  // M-step tile: bytes between 8-row groups of G^T
+constexpr uint32_t E_LBO = 144;    // E-step tile: bytes between the cores of a pair group
 
 enum Mode { ESTEP = 0, MSTEP = 1, PRED = 2 };
 
@@ -89,16 +110,24 @@ __host__ __device__ constexpr uint32_t idesc_tf32(int M, int N, int a_mn_major, 
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// One MMA by the lane elect.sync picks, in warp-uniform control flow: the
+// descriptors then stay in uniform registers and a rolled loop issues one MMA
+// every 62 cycles, as fast as the tensor cores take them at N = 128.  (Behind an
+// `if (lane == 0)` a rolled loop takes 89 and an unrolled one, too large to stay
+// in the instruction cache beside the other roles, up to 300.)
 __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
       "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
+// Completion of the elected lane's MMAs so far on mbar.
 __device__ __forceinline__ void commit(uint64_t *mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
-               : "memory");
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(mbar))
+      : "memory");
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
@@ -121,7 +150,8 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 
 // Waits for the phase with the given parity; false once kWaitLimitNs have
-// passed (checked every 1024 polls) or after kSpinLimit polls.
+// passed since the 64th poll (checked every 1024 polls) or after kSpinLimit
+// polls.  The global timer is not read on the way of a short wait.
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity) {
   const uint32_t addr = smem_u32(mbar);
   uint64_t t0 = 0;
@@ -134,26 +164,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity) {
         : "r"(addr), "r"(parity)
         : "memory");
     if (done) return true;
-    if ((it & 1023u) == 0) {
+    if ((it & 1023u) == 63u) {
       const uint64_t now = global_ns();
-      if (it == 0) t0 = now;
+      if (it == 63u) t0 = now;
       else if (now - t0 > kWaitLimitNs) return false;
     }
   }
   return false;
 }
-
-// Global -> shared bulk copy completing on mbar (16-byte aligned addresses, size a multiple of 16).
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint64_t *mbar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(smem_u32(mbar))
-               : "memory");
-}
-
-__device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -169,47 +187,40 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// 16 consecutive fp32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
+// 16 consecutive fp32 columns of this thread's TMEM lane (valid after tmem_wait).
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15}, [%16];\n"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Orders the uses of loaded registers after tmem_wait.
+__device__ __forceinline__ void tmem_use(uint32_t (&r)[16]) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]));
 }
 
-// 16 consecutive fp32 columns at each of two TMEM addresses of this thread's
-// lane, one wait for both.
-__device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, float (&v)[16], float (&u)[16]) {
-  uint32_t r[16], q[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(ta));
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];\n"
-      : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
-        "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
-      : "r"(tb));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    v[i] = __uint_as_float(r[i]);
-    u[i] = __uint_as_float(q[i]);
-  }
+// 16 bytes of a pair row (read once by this SM, so not kept in L1).
+__device__ __forceinline__ float4 ldg_row(const float *p) {
+  float4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p));
+  return v;
 }
 
-__device__ __forceinline__ void split4(const float4 x, float4 &hi, float4 &lo) {
-  hi = make_float4(tf32_rna(x.x), tf32_rna(x.y), tf32_rna(x.z), tf32_rna(x.w));
-  lo = make_float4(tf32_rna(x.x - hi.x), tf32_rna(x.y - hi.y), tf32_rna(x.z - hi.z), tf32_rna(x.w - hi.w));
+// The same under a predicate, v kept otherwise: the load is issued into v itself
+// (behind an `if` the compiler loads a temporary and selects, which waits for
+// the load: a thousand cycles per tile).
+__device__ __forceinline__ void ldg_row_if(bool ok, const float *p, float4 &v) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+      "@q ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+      : "l"(p), "r"((int)ok));
 }
 
 // Float offset of segment J of a W-core block (segments J' < J hold NT - J'
@@ -235,141 +246,133 @@ struct Args {
   float *SPo;            // ... or the S halves of the interleaved S / P tiles
   float *nu_out;         // M-step output
   float nu0;
-  float *ws_m, *ws_s;    // predictive density partials [gridDim.x, Nq]
-  int64_t Nq, q0, qn, chunk;
-  int64_t npts;          // rows of X (pair points) or of Y (queries)
+  float *ws_m, *ws_s;    // predictive density partials [gridDim.x / nqb, Nq]
+  int64_t Nq, nqb, chunk;  // predictive density: queries, blocks of QB queries, kernels per CTA
+  int64_t npts;          // rows of X (pair points)
   int64_t N;
   int64_t koff;          // row n is the kernel centred on X[n + koff]
   int D;
   int nt;                // 8-row blocks of the tiled layouts (W cores, SP)
   int ntile;             // nt (nt + 1) / 2
   int32_t *queue;        // row counter of the work queue (zero at launch), or null
+  int batch;             // rows per claim, at most 32
   int32_t *err;
-  int stall;             // test hook: the first stage expects 16 bytes no copy delivers
+  int stall;             // test hook: the first W copy expects 16 bytes no copy delivers
 };
 
-// Shared memory of one CTA.  The E-step and the predictive density keep two
-// A tiles that take the gathered pair rows in place (the MMAs of one tile
-// run while the other is converted); the M-step transposes, so its rows
-// land in two raw stages and it converts into one tile.  The B stages of
-// the E-step / predictive density are the accumulator copy of the M-step's
-// epilogue.
-template <int MODE>
-struct SmemL {
-  static constexpr bool DUAL = MODE != MSTEP;
-  static constexpr uint32_t TILE_BYTES = DUAL ? 65536u : 16u * GT_SBO;   // M-step: 16 x GT_SBO
-  static constexpr uint32_t TILE = 0;                                   // 2 (M-step: 1) A tiles
-  static constexpr uint32_t RAW = TILE + (DUAL ? 2 : 1) * TILE_BYTES;   // M-step: 2 x 34 KB
-  static constexpr uint32_t BST = RAW + (DUAL ? 0 : 2 * MT * RAW_STRIDE);  // 2 x (hi 16 KB + lo 16 KB)
-  static constexpr uint32_t B_BYTES = 16384;
-  static constexpr uint32_t RSTR = 68;                                  // M-step accumulator copy row stride
-  static constexpr uint32_t RED = BST;
-  static constexpr uint32_t XN = BST + 4 * B_BYTES;                     // NS x 256 B kernel centres
-  static constexpr uint32_t CIDX = XN + NS * 256;                       // NS x 128 int
-  static constexpr uint32_t RV = CIDX + NS * MT * 4;                    // NS x 128 float
-  static constexpr uint32_t META = RV + NS * MT * 4;                    // NS x Meta
-  static constexpr uint32_t PM = META + NS * 64;                        // predictive density (max, sum)
-  static constexpr uint32_t BAR = PM + 2 * PQ * 4;                      // mbarriers
-  static constexpr uint32_t bytes = BAR + 256;
-};
-static_assert(SmemL<MSTEP>::RSTR * 128 * 4 <= 4 * SmemL<MSTEP>::B_BYTES, "accumulator copy fits the B stages");
-static_assert(SmemL<MSTEP>::bytes + 1024 <= 232448 && SmemL<ESTEP>::bytes + 1024 <= 232448,
-              "shared memory of one CTA");
-
-// mbarriers (8 bytes each from SmemL::BAR)
-struct Bars {
-  static constexpr int MFULL = 0;          // [NS] metadata of a slot written (32 producer lanes)
-  static constexpr int MEMPTY = NS;        // [NS] slot free again (consumer thread 0)
-  static constexpr int RFULL = 2 * NS;     // [2] pair rows and kernel centre landed (64 gatherer lanes + 1)
-  static constexpr int REMPTY = RFULL + 2; // [2] rows' buffer free: M-step raw stage converted, else A tile's MMAs done
-  static constexpr int BFULL = REMPTY + 2; // [2] W cores of a B stage landed
-  static constexpr int BEMPTY = BFULL + 2; // [2] MMAs of the stage's last row done (tcgen05.commit)
-  static constexpr int MMA = BEMPTY + 2;   // [2] MMAs of tile t done (t % 2; tcgen05.commit)
-  static constexpr int CONV = MMA + 2;     // [2] tile t converted (t % 2; every consumer thread)
-  static constexpr int COUNT = CONV + 2;
-};
-static_assert(Bars::COUNT * 8 <= 256, "mbarrier area");
-
-struct Meta {
-  int64_t n;      // kernel row (< 0: no more tiles)
-  int64_t base;   // first pair of the tile (CSR position; predictive density: query offset in the block)
-  int cnt;        // pairs in the tile
-  int flags;      // 1: first tile of its row, 2: last tile, 4: row has an invalid index, 8: B stage used before
-  int bs;         // B stage / accumulator of the row (row counter parity)
-  int bph;        // parity of this row's use of B stage bs (its W-copy mbarrier phase)
-  float c0, c1;   // E-step: 0.5 E[log|Lambda|], -nu / 2;  predictive density: log coefficient, (nu + 1) / 2
-  float rsum;     // M-step: sum of r over the row (last tile)
-};
-
-// All 32 lanes of a warp AND-reduce v over the n threads of named barrier id.
-__device__ __forceinline__ bool bar_and(int id, int n, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
-}
-
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-
+// Shape, shared memory and residency of one instantiation.
 template <int MODE, int DP>
-struct Kern {
-  using Smem = SmemL<MODE>;
-  static constexpr int NCH = DP / 4;     // 4-dim chunks of a row
-  static constexpr int HCH = NCH / 2;    // chunks per converter thread
+struct Cfg {
+  static constexpr int NCH = DP / 4;                          // 16-byte chunks of a padded row
+  static constexpr int LPR = NCH <= 4 ? 4 : NCH <= 8 ? 8 : 16;  // lanes per row
+  static constexpr int RW = 32 / LPR;                         // rows (M-step: pair quads) per warp instruction
+  // converter and epilogue warps (eight of each an SM).  Sixteen converters
+  // were slower: they and the MMAs, which read 128 bytes of shared memory a
+  // cycle, wait for one another
+  static constexpr int NCW = DP <= 32 && MODE != PRED ? 4 : 8, NEW = DP <= 32 ? 4 : 8, NGRP = NEW / 4;
+  static constexpr int THREADS = 32 * (NCW + NEW + 2 + (MODE == MSTEP ? 0 : NCOPY) + (MODE == PRED ? 0 : NIDX));
+  static constexpr int NP = MT / (NCW * RW);                  // rows per consumer thread
+  static constexpr int NU = (MT / 4 + NCW * RW - 1) / (NCW * RW);  // M-step: pair quads per consumer thread
+  // two CTAs an SM below 48 dimensions, with one A tile each in the M-step
+  // (65 KB at every D); two A tiles otherwise
+  static constexpr int CTAS = DP <= 32 ? 2 : 1;
+  static constexpr int NA = (MODE == MSTEP && CTAS == 2) ? 1 : 2;
+  static constexpr uint32_t LO = NCH * E_LBO, SBO = 2 * NCH * E_LBO;
   // M-step accumulator columns: the hi rows 0..63 of G^T, then its lo rows
   // 64..64 + DP (rounded up to 16, the MMA's N granule)
   static constexpr int MN = 64 + ((DP + 15) / 16) * 16;
-  // TMEM columns of one accumulator (two are allocated): the M-step's
-  // [hi | lo] rows of G^T, the E-step's [hi | lo] output columns
-  static constexpr uint32_t ACC_COLS = 128u;
   static constexpr int NG = DP / 8;  // 8-row groups of one half of a B stage's K step
+  static constexpr int NTAB = NG * (NG + 1);  // 256-byte tiles of a row's W cores
+  // TMEM columns of one of the two accumulators (a power of two)
+  static constexpr uint32_t ACC = MODE == MSTEP ? 128u : DP <= 16 ? 32u : DP <= 32 ? 64u : 128u;
+  static constexpr uint32_t RSTR = DP + 4;  // M-step accumulator copy row stride (floats)
 
-  // ------------------------------------------------------- metadata warp
-  // State of the metadata warp.  Rows are fetched 32 at a time, lane j
-  // holding row j of the batch (its index, pair range and row constants:
-  // the dependent loads and the digamma sums of 32 rows run side by side);
-  // tiles are planned from the batch, and each tile's column indices and
-  // weights are loaded one tile before they are written.
-  struct Prod {
-    int64_t bn, ba, bb;  // this lane's batch row: kernel (-1: none) and pair range
-    float bc0, bc1;      // its row constants
-    int bsz, bidx;       // rows in the batch, next one to start
-    int64_t popped;      // row slots taken by this CTA
-    bool exhausted;      // no rows left to fetch
-    bool done;
-    int64_t n, next, end;  // current row and the first pair of its next tile
-    int rows;            // rows started (their parity selects the B stage / accumulator)
-    int bpar, bused;     // bit b: parity of the next use of B stage b, stage b used
+  static constexpr uint32_t TILE_BYTES = MODE == MSTEP ? 16u * GT_SBO : 16u * SBO;
+  static constexpr uint32_t B_BYTES = MODE == MSTEP ? 2u * DP * RSTR * 4u : (uint32_t)DP * DP * 8u;
+  static constexpr uint32_t TILE = 0;                       // NA A tiles
+  static constexpr uint32_t BST = TILE + NA * TILE_BYTES;   // 2 B stages (M-step: 2 accumulator copies)
+  static constexpr uint32_t CIDX = BST + 2 * B_BYTES;       // NS x 128 int
+  static constexpr uint32_t RV = CIDX + (MODE == PRED ? 0 : NS * MT * 4);  // M-step: NS x 128 float
+  static constexpr uint32_t RS = RV + (MODE == MSTEP ? NS * MT * 4 : 0);  // M-step: NS x (sum of r, invalid index)
+  static constexpr uint32_t META = RS + (MODE == MSTEP ? NS * 8 : 0);  // NPL x Meta
+  static constexpr uint32_t BAR = META + NPL * 64;          // mbarriers
+  static constexpr uint32_t TAB = BAR + 320;                // B-stage offset of each W-core tile
+  static constexpr uint32_t bytes = TAB + (MODE == MSTEP ? 0 : NTAB * 4);
+  static_assert(CTAS * (bytes + 2048) <= 233472, "shared memory of the resident CTAs");
+  static_assert(CTAS * 2 * ACC <= 512, "tensor memory of the resident CTAs");
+};
+
+// mbarriers (8 bytes each from Cfg::BAR)
+struct Bars {
+  static constexpr int PFULL = 0;          // [2] a half of the plan written (the planner)
+  static constexpr int PEMPTY = 2;         // [2] ... and its last tile done with (converter, epilogue and copy warps)
+  static constexpr int MFULL = 4;          // [NS] indices of a slot written (32 lanes of its index warp)
+  static constexpr int MEMPTY = MFULL + NS;  // [NS] slot free again (converter and epilogue warps)
+  static constexpr int BFULL = MEMPTY + NS;  // [2] W cores of a B stage landed (every copy-warp lane)
+  static constexpr int BEMPTY = BFULL + 2; // [2] MMAs of the stage's last row done (tcgen05.commit)
+  static constexpr int MMA = BEMPTY + 2;   // [2] MMAs of tile t done (t % 2; tcgen05.commit)
+  static constexpr int CONV = MMA + 2;     // [2] tile t converted (t % 2; every converter warp), and, but for the M-step,
+                                           // tile t - 2's accumulator read (its warpgroup)
+  static constexpr int EFULL = CONV + 2;   // [2] M-step: accumulator copy of warpgroup g written (its 4 warps)
+  static constexpr int EFREE = EFULL + 2;  // [2] ... and read
+  static constexpr int AFULL = EFREE + 2;  // [2] M-step: MMAs of a row's last tile done (row % 2; tcgen05.commit)
+  static constexpr int AFREE = AFULL + 2;  // [2] M-step: row's accumulator read (its warpgroup)
+  static constexpr int COUNT = AFREE + 2;
+};
+static_assert(Bars::COUNT * 8 <= 320, "mbarrier area");
+
+struct Meta {
+  int64_t base;   // first pair of the tile (CSR position; predictive density: query offset)
+  int64_t n;      // kernel row (< 0: no more tiles)
+  int cnt;        // pairs in the tile
+  int flags;      // 1: first tile of its row, 2: last tile, 4: the row's pair range is invalid
+  int row;        // rows started before (parity: B stage, M-step accumulator)
+  float c0, c1;   // E-step: 0.5 E[log|Lambda|], -nu / 2;  predictive density: log coefficient, (nu + 1) / 2
+};
+static_assert(sizeof(Meta) <= 64, "plan entry");
+
+template <int MODE, int DP>
+struct Kern {
+  using Smem = Cfg<MODE, DP>;
+  static constexpr int NG = Smem::NG;
+
+  static __device__ __forceinline__ Meta &meta_of(unsigned char *sm, int t) {
+    return *reinterpret_cast<Meta *>(sm + Smem::META + (t & (NPL - 1)) * 64);
+  }
+  static __device__ __forceinline__ const Meta &meta_of(const unsigned char *sm, int t) {
+    return *reinterpret_cast<const Meta *>(sm + Smem::META + (t & (NPL - 1)) * 64);
+  }
+
+  // ------------------------------------------------------- planner warp
+  // Rows are fetched up to 32 at a time, lane j holding row j of the batch: its
+  // kernel (n < 0: none), pair range and row constants (the dependent loads
+  // and the digamma sums of 32 rows run side by side), the number of tiles
+  // before it in the batch and of rows started before it.
+  struct Batch {
+    int64_t n, a, b;
     float c0, c1;
-    int rowbad;          // the current row's pair range is invalid
-    float racc;          // M-step: running sum of r over the row (at write time)
-    int bad;             // M-step: invalid index seen in the row (at write time)
+    int before, row, bad;
+    int tiles, next;  // tiles of the batch, next one to plan (uniform)
+    int64_t popped;   // row slots taken by this CTA (uniform)
+    int rows;         // rows started (uniform)
+    bool exhausted;   // no rows left to fetch (uniform)
   };
 
-  struct Plan {
-    int64_t n, base;
-    int cnt, flags, bs, bph;
-    float c0, c1;
-  };
-
-  // The next 32 row slots of this CTA: the work queue (an atomic counter
-  // over the caller's row order, 32 slots per claim), a static stride over
-  // the grid without a queue, or the CTA's contiguous chunk of kernels for the
-  // predictive density.  Valid slots are a prefix of the lanes.
-  static __device__ void fetch_batch(const Args &g, Prod &P, int lane) {
+  // The next row slots of this CTA: the work queue (an atomic counter over the
+  // caller's row order, `batch` slots per claim), a static stride over the grid
+  // without a queue (32 slots), or the CTA's contiguous chunk of kernels for
+  // the predictive density.  Valid slots are a prefix of the lanes.
+  static __device__ void fetch_batch(const Args &g, Batch &P, int lane) {
     int64_t it;
     bool valid = true;
     if (MODE == PRED) {
       valid = P.popped + lane < g.chunk;
-      it = (int64_t)blockIdx.x * g.chunk + P.popped + lane;
+      it = (int64_t)(blockIdx.x / g.nqb) * g.chunk + P.popped + lane;
     } else if (g.queue) {
       int v = 0;
-      if (lane == 0) v = atomicAdd(g.queue, 32);
+      if (lane == 0) v = atomicAdd(g.queue, g.batch);
       it = (int64_t)__shfl_sync(0xffffffffu, v, 0) + lane;
+      valid = lane < g.batch;
     } else {
       it = (int64_t)blockIdx.x + (P.popped + lane) * (int64_t)gridDim.x;
     }
@@ -383,7 +386,8 @@ struct Kern {
         a = g.rowptr[n];
         b = g.rowptr[n + 1];
       } else {
-        b = g.qn;
+        const int64_t left = g.Nq - (int64_t)(blockIdx.x % g.nqb) * QB;
+        b = left < QB ? left : QB;
       }
       if (MODE == ESTEP) {
         // 0.5 (psi_D(nu / 2) + D log 2 + logdet W), -nu / 2
@@ -397,110 +401,103 @@ struct Kern {
         c1 = 0.5f * (g.nu[n] + 1.f);
       }
     }
-    P.bn = n;
-    P.ba = a;
-    P.bb = b;
-    P.bc0 = c0;
-    P.bc1 = c1;
-    P.bsz = __popc(__ballot_sync(0xffffffffu, valid));
-    P.bidx = 0;
-    if (P.bsz < 32) P.exhausted = true;
+    const int got = __popc(__ballot_sync(0xffffffffu, valid));
+    if (got < (MODE != PRED && g.queue ? g.batch : 32)) P.exhausted = true;
+    P.n = n;
+    P.a = a;
+    P.bad = b < a;
+    P.b = b < a ? a : b;
+    P.c0 = c0;
+    P.c1 = c1;
+    // tiles of this lane's row: an E-step row without pairs has no log rho to
+    // write, an M-step row without pairs still gets one (empty) tile
+    int tiles = 0;
+    if (valid) {
+      const int64_t k = (P.b - a + MT - 1) / MT;
+      tiles = (int)(k < 1 && MODE != ESTEP ? 1 : k);
+    }
+    const unsigned started = __ballot_sync(0xffffffffu, tiles > 0);
+    P.row = P.rows + __popc(started & ((1u << lane) - 1u));
+    P.rows += __popc(started);
+    int incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    P.before = incl - tiles;
+    P.tiles = __shfl_sync(0xffffffffu, incl, 31);
+    P.next = 0;
   }
 
-  // Plans the next tile (n < 0: no work left).
-  static __device__ Plan plan_tile(const Args &g, Prod &P, int lane) {
-    Plan t{};
-    bool first = false;
-    if (!P.done && P.next >= P.end) {
-      for (;;) {
-        if (P.bidx >= P.bsz) {
-          if (P.exhausted) {
-            P.done = true;
-            break;
-          }
-          fetch_batch(g, P, lane);
-          continue;
+  // Plans tiles t0 .. t0 + 31 (one per lane; fewer, then the stop marker, at the
+  // end).  False once the marker is written.
+  static __device__ bool plan_half(const Args &g, Batch &P, unsigned char *sm, int t0, int lane) {
+    int pos = 0;
+    while (pos < 32) {
+      if (P.next >= P.tiles) {
+        if (P.exhausted) {
+          if (lane == 0) meta_of(sm, t0 + pos).n = -1;
+          return false;
         }
-        const int j = P.bidx++;
-        const int64_t n = __shfl_sync(0xffffffffu, P.bn, j);
-        const int64_t a = __shfl_sync(0xffffffffu, P.ba, j);
-        const int64_t b = __shfl_sync(0xffffffffu, P.bb, j);
-        const float c0 = __shfl_sync(0xffffffffu, P.bc0, j);
-        const float c1 = __shfl_sync(0xffffffffu, P.bc1, j);
-        if (MODE == ESTEP && b <= a) continue;  // no pairs: no log rho to write
-        P.n = n;
-        P.next = a;
-        P.end = b < a ? a : b;  // an M-step row without pairs still gets one (empty) tile
-        P.rowbad = b < a;
-        P.c0 = c0;
-        P.c1 = c1;
-        first = true;
-        ++P.rows;
-        break;
+        fetch_batch(g, P, lane);
+        continue;
       }
+      const int take = min(32 - pos, P.tiles - P.next);
+      const int y = P.next + lane;
+      // the row of tile y: the last lane with before <= y (rows without tiles
+      // share their successor's)
+      int j = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, P.before, (j + o) & 31);
+        if (j + o < 32 && v <= y) j += o;
+      }
+      Meta m;
+      m.n = __shfl_sync(0xffffffffu, P.n, j);
+      const int64_t a = __shfl_sync(0xffffffffu, P.a, j), b = __shfl_sync(0xffffffffu, P.b, j);
+      const int k = y - __shfl_sync(0xffffffffu, P.before, j);
+      m.base = a + (int64_t)k * MT;
+      m.cnt = (int)(b - m.base < MT ? b - m.base : MT);
+      m.flags = (k == 0 ? 1 : 0) | (b - m.base <= MT ? 2 : 0) | (__shfl_sync(0xffffffffu, P.bad, j) ? 4 : 0);
+      m.row = __shfl_sync(0xffffffffu, P.row, j);
+      m.c0 = __shfl_sync(0xffffffffu, P.c0, j);
+      m.c1 = __shfl_sync(0xffffffffu, P.c1, j);
+      if (lane < take) meta_of(sm, t0 + pos + lane) = m;
+      pos += take;
+      P.next += take;
     }
-    if (P.done) {
-      t.n = -1;
-      return t;
-    }
-    t.n = P.n;
-    t.base = P.next;
-    t.cnt = (int)((P.end - P.next) < MT ? (P.end - P.next) : MT);
-    P.next += t.cnt;
-    const bool last = P.next >= P.end;
-    t.bs = (P.rows - 1) & 1;
-    t.bph = 0;
-    int reused = 0;
-    if (first) {
-      t.bph = (P.bpar >> t.bs) & 1;
-      reused = (P.bused >> t.bs) & 1;
-      P.bpar ^= 1 << t.bs;
-      P.bused |= 1 << t.bs;
-    }
-    t.flags = (first ? 1 : 0) | (last ? 2 : 0) | (P.rowbad ? 4 : 0) | (reused ? 8 : 0);
-    t.c0 = P.c0;
-    t.c1 = P.c1;
-    return t;
+    return true;
   }
 
-  // Issues the loads of a planned tile's column indices and weights (4 pairs
-  // per lane).
-  static __device__ __forceinline__ void load_tile(const Args &g, const Plan &t, int lane, int32_t (&c)[4],
+  // --------------------------------------------------------- index warps
+  // Loads the column indices and weights of a planned tile (4 pairs per lane).
+  static __device__ __forceinline__ void load_tile(const Args &g, const Meta &m, int lane, int32_t (&c)[4],
                                                    float (&w)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int p = lane + 32 * k;
       c[k] = -1;
       w[k] = 0.f;
-      if (t.n >= 0 && p < t.cnt) {
-        if (MODE == PRED) {
-          c[k] = (int32_t)(g.q0 + t.base + p);
-        } else {
-          c[k] = g.col[t.base + p];
-          if (MODE == MSTEP) w[k] = g.r[t.base + p];
-        }
+      if (p < m.cnt) {
+        c[k] = g.col[m.base + p];
+        if (MODE == MSTEP) w[k] = g.r[m.base + p];
       }
     }
   }
 
-  // Writes a planned tile (or the stop marker) into slot ms, validating its
-  // column indices, and arrives on mfull (every lane).
-  static __device__ void write_tile(const Args &g, Prod &P, const Plan &t, const int32_t (&c)[4],
-                                    const float (&w)[4], unsigned char *sm, uint64_t *mfull, int ms, int lane) {
-    Meta *meta = reinterpret_cast<Meta *>(sm + Smem::META) + ms;
-    if (t.n < 0) {
-      if (lane == 0) meta->n = -1;
-      mbar_arrive(mfull);
-      return;
-    }
+  // Writes them into slot ms, validated, and arrives on mfull (every lane).
+  // Brings a new row's W cores and kernel centre into L2: the slot is up to NS
+  // tiles ahead of the consumers.
+  static __device__ __forceinline__ void write_tile(const Args &g, const Meta &m, const int32_t (&c)[4],
+                                                    const float (&w)[4], unsigned char *sm, uint64_t *mfull, int ms,
+                                                    int lane) {
     int32_t *cidx = reinterpret_cast<int32_t *>(sm + Smem::CIDX) + ms * MT;
     float *rv = reinterpret_cast<float *>(sm + Smem::RV) + ms * MT;
-    const uint32_t rb = (uint32_t)(((g.D + 3) / 4) * 16);  // bytes per row
-    // this slot is up to NS - 2 tiles ahead of the converters: pull a new
-    // row's W cores and kernel centre into L2 now
-    if (MODE != PRED && lane == 0 && (t.flags & 1)) {
-      if (MODE == ESTEP) prefetch_l2(g.Wc + t.n * (int64_t)(g.ntile * 128), (uint32_t)g.ntile * 512u);
-      prefetch_l2(g.X + (t.n + g.koff) * g.ldx, rb);
+    if (MODE == ESTEP && (m.flags & 1)) {
+      const char *wc = reinterpret_cast<const char *>(g.Wc + m.n * (int64_t)(g.ntile * 128));
+      for (uint32_t o = lane * 128u; o < (uint32_t)g.ntile * 512u; o += 32u * 128u)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(wc + o));
     }
     unsigned bad = 0;
     float rs = 0.f;
@@ -509,7 +506,7 @@ struct Kern {
       const int p = lane + 32 * k;
       int32_t ck = c[k];
       float wk = w[k];
-      if (MODE != PRED && p < t.cnt && (ck < 0 || ck >= g.npts)) {
+      if (p < m.cnt && (ck < 0 || ck >= g.npts)) {
         ck = -1;
         wk = 0.f;
         bad = 1;
@@ -520,424 +517,401 @@ struct Kern {
         rs += wk;
       }
     }
-    int flags = t.flags;
     if (MODE == MSTEP) {
       bad = __reduce_or_sync(0xffffffffu, bad);
       rs = warp_sum(rs);
-      if (t.flags & 1) {
-        P.racc = 0.f;
-        P.bad = 0;
-      }
-      P.racc += rs;
-      P.bad |= (int)bad;
-      if (P.bad) flags |= 4;
-    }
-    if (lane == 0) {
-      meta->n = t.n;
-      meta->base = t.base;
-      meta->cnt = t.cnt;
-      meta->flags = flags;
-      meta->bs = t.bs;
-      meta->bph = t.bph;
-      meta->c0 = t.c0;
-      meta->c1 = t.c1;
-      meta->rsum = P.racc;
+      if (lane == 0)
+        reinterpret_cast<float2 *>(sm + Smem::RS)[ms] = make_float2(rs, __uint_as_float(bad));
     }
     mbar_arrive(mfull);
   }
 
-  // --------------------------------------------------------- gather warp
-  // The W cores of the row starting at the tile in slot ms into its B stage
-  // (the E-step and the predictive density), on mbarrier bfull.
-  static __device__ void copy_w(const Args &g, unsigned char *sm, const Meta &meta, uint64_t *bfull, int lane) {
-    const float *wsrc = g.Wc + meta.n * (int64_t)(g.ntile * 128);
-    unsigned char *bst = sm + Smem::BST + (uint32_t)meta.bs * 2 * Smem::B_BYTES;
-    if (lane == 0) mbar_arrive_tx(bfull, (uint32_t)g.ntile * 512u);
-    __syncwarp();
-    // per segment J: its hi tiles and its lo tiles, each run to its half of
-    // the K step's row groups
-    for (int J = lane; J < g.nt; J += 32) {
-      const uint32_t run = (uint32_t)(g.nt - J) * 256u;
-      const float *src = wsrc + wseg(J, g.nt);
-      bulk_g2s(smem_u32(bst + (J * 2 * NG + J) * 256), src, run, bfull);
-      bulk_g2s(smem_u32(bst + (J * 2 * NG + NG + J) * 256), src + (g.nt - J) * 64, run, bfull);
+  // ---------------------------------------------------------- copy warps
+  // B-stage offset of W-core tile x (256 bytes) of a row: segment J holds its
+  // hi tiles I = J .. nt - 1, then their lo tiles; K step J of the stage has 2
+  // NG row groups, hi then lo.
+  static __device__ uint32_t core_offset(int x, int nt) {
+    int J = 0;
+    while (x >= 2 * (nt - J)) x -= 2 * (nt - J++);
+    const int lo = x >= nt - J;
+    return (uint32_t)(J * 2 * NG + lo * NG + J + x - lo * (nt - J)) * 256u;
+  }
+
+  // The W cores of the row starting at the tile of `meta` into its B stage
+  // (the E-step and the predictive density): 512 contiguous bytes per warp
+  // instruction, the copy warps taking alternate ones.  (Sixteen bulk copies
+  // per row, a run each, took one warp 1.9k cycles to issue.)
+  static __device__ __forceinline__ void copy_w(const Args &g, unsigned char *sm, const Meta &meta, int cw, int lane) {
+    const unsigned char *src = reinterpret_cast<const unsigned char *>(g.Wc + meta.n * (int64_t)(g.ntile * 128));
+    const uint32_t *tab = reinterpret_cast<const uint32_t *>(sm + Smem::TAB);
+    const uint32_t bst = smem_u32(sm + Smem::BST + (uint32_t)(meta.row & 1) * Smem::B_BYTES) + (lane & 15) * 16u;
+    const int n2 = 2 * g.ntile;
+#pragma unroll 6
+    for (int x = 2 * cw + (lane >> 4); x < n2; x += 2 * NCOPY)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bst + tab[x]),
+                   "l"(src + (uint32_t)x * 256u + (lane & 15) * 16u)
+                   : "memory");
+  }
+
+  // ------------------------------------------------------- converter warps
+  // What a converter thread holds of the tile it converts next: chunk k (lane %
+  // LPR) of its rows, and of the kernel centre.
+  struct Rows {
+    float4 x[MODE == MSTEP ? 4 * Smem::NU : Smem::NP];
+    float4 c;
+  };
+
+  // Bit masks of the tf32 rounding per dim of chunk k: zero beyond D, where a
+  // row's padding may hold anything.
+  static __device__ __forceinline__ uint4 dim_masks(int k, int D) {
+    const int d0 = 4 * k;
+    const uint32_t m = 0xFFFFE000u;
+    return make_uint4(m, d0 + 1 < D ? m : 0u, d0 + 2 < D ? m : 0u, d0 + 3 < D ? m : 0u);
+  }
+  static __device__ __forceinline__ float rna(float x, uint32_t m) {
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & m);
+  }
+
+  // E-step / predictive density: row p of the tile's operand from x - c, split
+  // as tf32 hi + lo.
+  static __device__ __forceinline__ void store_row(unsigned char *tile, int p, int k, float4 x, float4 c, uint4 m) {
+    const float4 d = make_float4(x.x - c.x, x.y - c.y, x.z - c.z, x.w - c.w);
+    const float4 hi = make_float4(rna(d.x, m.x), rna(d.y, m.y), rna(d.z, m.z), rna(d.w, m.w));
+    const float4 lo = make_float4(rna(d.x - hi.x, m.x), rna(d.y - hi.y, m.y), rna(d.z - hi.z, m.z),
+                                  rna(d.w - hi.w, m.w));
+    unsigned char *o = tile + (uint32_t)(p >> 3) * Smem::SBO + (uint32_t)k * E_LBO + (uint32_t)(p & 7) * 16u;
+    *reinterpret_cast<float4 *>(o) = hi;
+    *reinterpret_cast<float4 *>(o + Smem::LO) = lo;
+  }
+
+  // Loads the rows of tile t.  Issued after the previous tile's conversion was
+  // handed over: fence.proxy.async waits for the loads in flight (issuing each
+  // as its register came free put their whole latency on every tile).
+  static __device__ __forceinline__ void load_rows(const Args &g, const unsigned char *sm, int t, int warp, int lane,
+                                                   Rows &R) {
+    const Meta &m = meta_of(sm, t);
+    const int k = lane & (Smem::LPR - 1), sub = lane / Smem::LPR;
+    if (k >= (g.D + 3) / 4) return;
+    ldg_row_if(true, g.X + (m.n + (MODE == PRED ? 0 : g.koff)) * g.ldx + 4 * k, R.c);
+    const int32_t *cidx = reinterpret_cast<const int32_t *>(sm + Smem::CIDX) + (t % NS) * MT;
+    const int cnt = m.cnt;
+    if (MODE == ESTEP) {
+      int32_t c[Smem::NP];
+#pragma unroll
+      for (int i = 0; i < Smem::NP; ++i) {
+        const int p = (i * Smem::NCW + warp) * Smem::RW + sub;
+        c[i] = p < cnt ? cidx[p] : -1;
+      }
+#pragma unroll
+      for (int i = 0; i < Smem::NP; ++i)
+        ldg_row_if(c[i] >= 0, g.X + (int64_t)c[i] * g.ldx + 4 * k, R.x[i]);
+    } else if (MODE == MSTEP) {
+#pragma unroll
+      for (int u = 0; u < Smem::NU; ++u) {
+        const int q = (u * Smem::NCW + warp) * Smem::RW + sub;
+        int4 c4 = make_int4(-1, -1, -1, -1);
+        if (4 * q < cnt) c4 = reinterpret_cast<const int4 *>(cidx)[q];
+        const int cs[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          R.x[4 * u + v] = make_float4(0.f, 0.f, 0.f, 0.f);
+          ldg_row_if(cs[v] >= 0, g.X + (int64_t)cs[v] * g.ldx + 4 * k, R.x[4 * u + v]);
+        }
+      }
     }
   }
 
-  // The pair (query) rows of the tile in slot ms into raw stage s, and its
-  // kernel centre into the slot's centre buffer, completing on mbarrier
-  // rfull (32 NGW + 1 arrivals: the byte count for the bulk copy, then one
-  // per lane of every gather warp when its cp.async copies have landed).  Half-warp h
-  // of gather warp gw copies the row groups 4 (4 j + 2 gw + h) .. + 3, lane
-  // k % 16 the 16-byte chunk k of each row: two 256-byte rows per
-  // instruction, the group's four column indices read as one 16-byte word,
-  // four groups in flight.
-  static __device__ __forceinline__ void gather(const Args &g, unsigned char *sm, const Meta &meta, int s, int ms,
-                                                uint64_t *rfull, bool stall, int gw, int lane) {
-    const uint32_t rb = (uint32_t)(((g.D + 3) / 4) * 16);  // bytes per row
-    if (gw == 0 && lane == 0) {
-      mbar_arrive_tx(rfull, rb + (stall ? 16u : 0u));  // a stalled stage expects 16 bytes no copy delivers
-      const float *xsrc = g.X + (meta.n + (MODE == PRED ? 0 : g.koff)) * g.ldx;
-      bulk_g2s(smem_u32(sm + Smem::XN + ms * 256), xsrc, rb, rfull);
-    }
-    const int64_t ld = (MODE == PRED) ? g.ldy : g.ldx;
-    const int cnt = meta.cnt;
-    if (Smem::DUAL) {
-      // straight into A tile s: chunk k of pair p at its hi slot (core (p / 8,
-      // k), row p % 8); lane (p % 8, k % 4), so a warp instruction fills four
-      // whole cores of one 8-pair group; gather warp gw takes the groups
-      // gw, gw + NGW, ...
-      const int32_t *cidx = reinterpret_cast<const int32_t *>(sm + Smem::CIDX) + ms * MT;
-      const uint32_t tb = smem_u32(sm + Smem::TILE + (uint32_t)s * Smem::TILE_BYTES);
-      const int pl = lane & 7, kk = lane >> 3;
-      const int rch = (g.D + 3) / 4;
-      const float *base = (MODE == PRED) ? g.Y : g.X;
-      for (int grp = gw; grp < MT / 8; grp += NGW) {
-        if (8 * grp >= cnt) break;
-        const int p = 8 * grp + pl;
-        const int32_t c = (p < cnt) ? cidx[p] : -1;
-        const float *src = base + (int64_t)(c < 0 ? 0 : c) * ld;
+  // Converts tile t (rows in R) into A tile `tile`.
+  static __device__ __forceinline__ void convert(const Args &g, unsigned char *sm, unsigned char *tile, int t,
+                                                 int warp, int lane, const Rows &R) {
+    const int k = lane & (Smem::LPR - 1), sub = lane / Smem::LPR;
+    if (k >= (g.D + 3) / 4) return;  // a chunk beyond D: its cores stay zero
+    const int cnt = meta_of(sm, t).cnt;
+    const uint4 mask = dim_masks(k, g.D);
+    const float4 c = R.c;
+    if (MODE == ESTEP) {
+      // rows past the tile's end are not stored: their accumulator lanes are
+      // not read
 #pragma unroll
-        for (int kq = 0; kq < NCH / 4; ++kq) {
-          const int k = 4 * kq + kk;
-          if (c >= 0 && k < rch)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tb + (uint32_t)grp * 4096u +
-                                                                              (uint32_t)k * 128u + (uint32_t)pl * 16u),
-                         "l"(src + 4 * k)
-                         : "memory");
-        }
+      for (int i = 0; i < Smem::NP; ++i) {
+        const int p = (i * Smem::NCW + warp) * Smem::RW + sub;
+        if (p < cnt) store_row(tile, p, k, R.x[i], c, mask);
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(rfull)) : "memory");
-      return;
-    }
-    const int4 *cid4 = reinterpret_cast<const int4 *>(sm + Smem::CIDX + ms * MT * 4);
-    const int h = lane >> 4, k = lane & 15;
-    const bool kin = 16 * k < (int)rb;
-    const uint32_t dst0 = smem_u32(sm + Smem::RAW + (uint32_t)s * MT * RAW_STRIDE) + 16u * k;
-    const float *base = ((MODE == PRED) ? g.Y : g.X) + 4 * k;
-#pragma unroll 4
-    for (int j = 0; j < MT / (8 * NGW); ++j) {
-      const int grp = 2 * NGW * j + 2 * gw + h;
-      if (4 * grp >= cnt) break;
-      const int4 c4 = cid4[grp];
-      const int cs[4] = {c4.x, c4.y, c4.z, c4.w};
+    } else {
+      // G^T: the quad's 4 pairs of dims 4 k .. 4 k + 3 as sqrt(r) (x_m - x_n),
+      // written per dim as one 16-byte row of a core, hi at row d, lo at row
+      // 64 + d.  Quads past the last 8-pair group are not multiplied.
+      const float4 *rv = reinterpret_cast<const float4 *>(sm + Smem::RV + (t % NS) * MT * 4);
+      const int nq = 2 * ((cnt + 7) / 8);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int p = 4 * grp + u;
-        if (kin && p < cnt && cs[u] >= 0)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + (uint32_t)p * RAW_STRIDE),
-                       "l"(base + (int64_t)cs[u] * ld)
-                       : "memory");
-      }
-    }
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(rfull)) : "memory");
-  }
-
-  // --------------------------------------------------------------- converter
-  static __device__ __forceinline__ void convert(const Args &g, unsigned char *sm, int s, int ms, int tid) {
-    const Meta &meta = reinterpret_cast<const Meta *>(sm + Smem::META)[ms];
-    const int32_t *cidx = reinterpret_cast<const int32_t *>(sm + Smem::CIDX) + ms * MT;
-    const float *rv = reinterpret_cast<const float *>(sm + Smem::RV) + ms * MT;
-    const unsigned char *raw = sm + Smem::RAW + (uint32_t)s * MT * RAW_STRIDE;
-    const float4 *xn = reinterpret_cast<const float4 *>(sm + Smem::XN + ms * 256);
-    unsigned char *tile = sm + Smem::TILE;
-    const int D = g.D;
-    const int rch = (D + 3) / 4;  // chunks present in a staged row
-    if (MODE == MSTEP) {
-      // G^T: unit (pair quad q, dim chunk k) reads the chunk of its 4 pairs
-      // (consecutive units: consecutive chunks, distinct bank groups), forms
-      // sqrt(r) (x_m - x_n), and writes per dim the 4 pairs as one 16-byte
-      // row of a core, hi at row d, lo at row 64 + d.  Both units' loads are
-      // issued before any store.
-      const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 xs[2][4], ccs[2];
-      float ws[2][4];
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {
-        const int u = tid + NTHR * s2;
-        const int q = u >> 4, k = u & 15;
-        ccs[s2] = (k < rch) ? xn[k] : z4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int p = 4 * q + i;
-          const bool ok = p < meta.cnt && k < rch && cidx[p] >= 0;
-          ws[s2][i] = ok ? rv[p] : 0.f;
-          xs[s2][i] = ok ? *reinterpret_cast<const float4 *>(raw + p * RAW_STRIDE + k * 16) : z4;
-        }
-      }
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {
-        const int u = tid + NTHR * s2;
-        const int q = u >> 4, k = u & 15;
-        const float4 cc = ccs[s2];
-        const int d0 = 4 * k;
+      for (int u = 0; u < Smem::NU; ++u) {
+        const int q = (u * Smem::NCW + warp) * Smem::RW + sub;
         float4 dq[4];
+        if (q < nq) {
+          const float4 w4 = rv[q];
+          const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = xs[s2][i];
-          const float w = ws[s2][i];
-          float4 d;
-          d.x = (x.x - cc.x) * w;
-          d.y = (d0 + 1 < D) ? (x.y - cc.y) * w : 0.f;
-          d.z = (d0 + 2 < D) ? (x.z - cc.z) * w : 0.f;
-          d.w = (d0 + 3 < D) ? (x.w - cc.w) * w : 0.f;
-          dq[i] = d;
+          for (int v = 0; v < 4; ++v) {
+            const bool in = 4 * q + v < cnt;
+            const float4 x = R.x[4 * u + v];
+            dq[v] = in ? make_float4((x.x - c.x) * w[v], (x.y - c.y) * w[v], (x.z - c.z) * w[v], (x.w - c.w) * w[v])
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
+        if (q < nq) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 v = j == 0   ? make_float4(dq[0].x, dq[1].x, dq[2].x, dq[3].x)
-                           : j == 1 ? make_float4(dq[0].y, dq[1].y, dq[2].y, dq[3].y)
-                           : j == 2 ? make_float4(dq[0].z, dq[1].z, dq[2].z, dq[3].z)
-                                    : make_float4(dq[0].w, dq[1].w, dq[2].w, dq[3].w);
-          float4 hi, lo;
-          split4(v, hi, lo);
-          const int r = 4 * k + j;
-          unsigned char *o = tile + (uint32_t)(r >> 3) * GT_SBO + (uint32_t)q * 128u + (uint32_t)(r & 7) * 16u;
-          *reinterpret_cast<float4 *>(o) = hi;
-          *reinterpret_cast<float4 *>(o + 8 * GT_SBO) = lo;
+          for (int j = 0; j < 4; ++j) {
+            const float4 v = j == 0   ? make_float4(dq[0].x, dq[1].x, dq[2].x, dq[3].x)
+                             : j == 1 ? make_float4(dq[0].y, dq[1].y, dq[2].y, dq[3].y)
+                             : j == 2 ? make_float4(dq[0].z, dq[1].z, dq[2].z, dq[3].z)
+                                      : make_float4(dq[0].w, dq[1].w, dq[2].w, dq[3].w);
+            const uint32_t mj = j == 0 ? mask.x : j == 1 ? mask.y : j == 2 ? mask.z : mask.w;
+            const float4 hi = make_float4(rna(v.x, mj), rna(v.y, mj), rna(v.z, mj), rna(v.w, mj));
+            const float4 lo = make_float4(rna(v.x - hi.x, mj), rna(v.y - hi.y, mj), rna(v.z - hi.z, mj),
+                                          rna(v.w - hi.w, mj));
+            const int r = 4 * k + j;
+            unsigned char *o = tile + (uint32_t)(r >> 3) * GT_SBO + (uint32_t)q * 128u + (uint32_t)(r & 7) * 16u;
+            *reinterpret_cast<float4 *>(o) = hi;
+            *reinterpret_cast<float4 *>(o + 8 * GT_SBO) = lo;
+          }
         }
-      }
-      return;
-    }
-    // in place: the gathered row chunk sits in its hi slot of A tile s
-    const int p = tid & (MT - 1), h = tid >> 7;
-    const int cvalid = (p < meta.cnt) ? cidx[p] : -1;
-    unsigned char *dst = tile + (uint32_t)s * Smem::TILE_BYTES + (uint32_t)(p >> 3) * 4096u + (uint32_t)(p & 7) * 16u;
-    // four chunks at a time: all their loads before any store (the stores
-    // into the tile would otherwise order the next loads behind them)
-#pragma unroll
-    for (int i0 = 0; i0 < HCH; i0 += 4) {
-      float4 x[4], c[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int k = h * HCH + i0 + i;
-        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        c[i] = x[i];
-        if (i0 + i < HCH && cvalid >= 0 && k < rch) {
-          x[i] = *reinterpret_cast<const float4 *>(dst + k * 128);
-          c[i] = xn[k];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int k = h * HCH + i0 + i;
-        if (i0 + i >= HCH) continue;
-        const int d0 = 4 * k;
-        float4 d;
-        d.x = x[i].x - c[i].x;
-        d.y = (d0 + 1 < D) ? x[i].y - c[i].y : 0.f;
-        d.z = (d0 + 2 < D) ? x[i].z - c[i].z : 0.f;
-        d.w = (d0 + 3 < D) ? x[i].w - c[i].w : 0.f;
-        float4 hi, lo;
-        split4(d, hi, lo);
-        *reinterpret_cast<float4 *>(dst + k * 128) = hi;
-        *reinterpret_cast<float4 *>(dst + 2048 + k * 128) = lo;
       }
     }
   }
 
   // ---------------------------------------------------------------- MMAs
-  static __device__ __forceinline__ void issue_mma(const Args &g, unsigned char *sm, const Meta &meta, uint32_t tmem,
-                                                   uint32_t acc_sel, int s, uint64_t *mma_done) {
-    const uint32_t tile = smem_u32(sm + Smem::TILE + (Smem::DUAL ? (uint32_t)s * Smem::TILE_BYTES : 0u));
+  static __device__ __forceinline__ void issue_mma(const Args &g, unsigned char *sm, int cnt, int first, int row,
+                                                   uint32_t tmem, int acc_sel, int a_tile, uint64_t *mma_done) {
+    const uint32_t tile = smem_u32(sm + Smem::TILE + (uint32_t)a_tile * Smem::TILE_BYTES);
+    const uint32_t td = tmem + (uint32_t)acc_sel * Smem::ACC;
     if (MODE == MSTEP) {
       // [G_hi; G_lo]^T [G_hi, G_lo] over the tile's pairs, 8 per MMA: the
       // four blocks hh, hl, lh, ll of (G_hi + G_lo)^T (G_hi + G_lo)
-      const uint32_t idesc = idesc_tf32(128, MN, 0, 0);
-      const uint32_t td = tmem + acc_sel * ACC_COLS;
-      const int ng = (meta.cnt + 7) / 8;
+      const uint32_t idesc = idesc_tf32(128, Smem::MN, 0, 0);
+      const int ng = (cnt + 7) / 8;
+      uint64_t d = desc(tile, 128, GT_SBO);
+      uint32_t acc = first ? 0u : 1u;
+#pragma unroll 1
       for (int gi = 0; gi < ng; ++gi) {
-        const uint32_t a = tile + (uint32_t)gi * 256u;
-        const uint32_t acc = ((meta.flags & 1) && gi == 0) ? 0u : 1u;
-        mma_tf32(td, desc(a, 128, GT_SBO), desc(a, 128, GT_SBO), idesc, acc);
+        mma_tf32(td, d, d, idesc, acc);
+        d += 16;
+        acc = 1u;
       }
     } else {
       // [D_hi; D_lo] [W_hi | W_lo] per K step: output columns 0..DP-1 take
       // the products with W_hi, DP..2 DP-1 those with W_lo (all four hi / lo
       // products; the epilogue adds the halves)
       const uint32_t idesc = idesc_tf32(128, 2 * DP, 0, 0);
-      const uint32_t td = tmem + acc_sel * ACC_COLS;
-      const uint32_t bst = smem_u32(sm + Smem::BST + (uint32_t)meta.bs * 2 * Smem::B_BYTES);
+      uint64_t a = desc(tile, E_LBO, Smem::SBO);
+      uint64_t b = desc(smem_u32(sm + Smem::BST + (uint32_t)(row & 1) * Smem::B_BYTES), 128, 256);
       const int nt = g.nt;
+#pragma unroll 1
       for (int J = 0; J < nt; ++J) {
-        const uint32_t ao = (uint32_t)J * 256u, bo = (uint32_t)(J * 2 * NG * 256);
-        mma_tf32(td, desc(tile + ao, 128, 4096), desc(bst + bo, 128, 256), idesc, J > 0);
-        mma_tf32(td, desc(tile + 2048 + ao, 128, 4096), desc(bst + bo, 128, 256), idesc, 1);
+        mma_tf32(td, a, b, idesc, J > 0);
+        mma_tf32(td, a + Smem::LO / 16, b, idesc, 1);
+        a += 2 * E_LBO / 16;
+        b += 2 * NG * 16;
       }
     }
     commit(mma_done);
   }
 
   // ---------------------------------------------------------------- epilogue
-  static __device__ void epilogue(const Args &g, unsigned char *sm, int ms, uint32_t tmem, uint32_t acc_sel,
-                                  int tid) {
-    const Meta &meta = reinterpret_cast<const Meta *>(sm + Smem::META)[ms];
-    const int32_t *cidx = reinterpret_cast<const int32_t *>(sm + Smem::CIDX) + ms * MT;
-    const int warp = tid >> 5;
-    if (MODE == MSTEP) {
-      if (!(meta.flags & 2)) return;
-      // accumulator row i < 64 holds (hh_ij, hl_ij) in columns (j, 64 + j),
-      // row 64 + i holds (lh_ij, ll_ij): each thread adds its row's two
-      // halves into shared memory, then S_ij = red_ij + red_(64+i)j over the
-      // lower triangle
-      float *red = reinterpret_cast<float *>(sm + Smem::RED);
-      const bool empty = (meta.cnt == 0) && (meta.flags & 1);
-      {
-        // warps w and w + 4 read the same 32 TMEM lanes, alternate 16-column blocks
-        const int row = tid & 127, half = tid >> 7;
-        const uint32_t taddr = tmem + acc_sel * ACC_COLS + ((uint32_t)((warp & 3) * 32) << 16);
-#pragma unroll
-        for (int cb = 0; cb < (DP + 15) / 16; ++cb) {
-          if ((cb & 1) != half) continue;
-          const int c0 = 16 * cb;
-          float v[16], u[16];
-          if (!empty) {
-            tmem_ld16x2(taddr + c0, taddr + 64 + c0, v, u);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = u[k] = 0.f;
-          }
-#pragma unroll
-          for (int k = 0; k < 16; k += 4)
-            *reinterpret_cast<float4 *>(red + row * Smem::RSTR + c0 + k) =
-                make_float4(v[k] + u[k], v[k + 1] + u[k + 1], v[k + 2] + u[k + 2], v[k + 3] + u[k + 3]);
-        }
-      }
-      fence_before();
-      asm volatile("bar.sync 1, %0;" ::"n"(NTHR) : "memory");
-      const int64_t n = meta.n;
-      const bool bad = (meta.flags & 4) != 0;
-      const int D = g.D;
-      const float *Uh = red, *Vl = red + 64 * Smem::RSTR;
-      if (tid == 0) g.nu_out[n] = bad ? NAN : g.nu0 + meta.rsum;
-      if (g.SPo) {
-        // four consecutive columns of one tile row per store: tile t = I (I +
-        // 1) / 2 + J (I from the root of 8 t + 1, exact at these sizes), row
-        // r = e / 2, columns 8 J + 4 (e % 2) + 0..3
-        float *dst = g.SPo + n * (int64_t)(g.ntile * 128);
-        for (int q = tid; q < g.ntile * 16; q += NTHR) {
-          const int t = q >> 4, e = q & 15;
-          const int I = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-          const int J = t - I * (I + 1) / 2;
-          const int i = 8 * I + (e >> 1), j = 8 * J + 4 * (e & 1);
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (i < D) {
-            const float4 a = *reinterpret_cast<const float4 *>(Vl + i * Smem::RSTR + j);
-            const float4 b = *reinterpret_cast<const float4 *>(Uh + i * Smem::RSTR + j);
-            v.x = (j <= i) ? a.x + b.x : 0.f;
-            v.y = (j + 1 <= i) ? a.y + b.y : 0.f;
-            v.z = (j + 2 <= i) ? a.z + b.z : 0.f;
-            v.w = (j + 3 <= i) ? a.w + b.w : 0.f;
-          }
-          if (bad) v = make_float4(NAN, NAN, NAN, NAN);
-          *reinterpret_cast<float4 *>(dst + t * 128 + (e >> 1) * 8 + 4 * (e & 1)) = v;
-        }
-      } else {
-        float *Sn = g.S + n * (int64_t)D * D;
-        for (int q = tid; q < D * D; q += NTHR) {
-          const int i = q / D, j = q % D;
-          if (g.lower_only && j > i) continue;
-          const int a = i > j ? i : j, b = i > j ? j : i;  // symmetric: from the lower triangle
-          Sn[q] = bad ? NAN : Vl[a * Smem::RSTR + b] + Uh[a * Smem::RSTR + b];
-        }
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(NTHR) : "memory");
-      return;
-    }
-    if (tid >= 128) return;
-    // lane = pair (query) row
-    const uint32_t taddr = tmem + acc_sel * ACC_COLS + ((uint32_t)(warp * 32) << 16);
+  // E-step / predictive density: Q of this thread's pair (TMEM lane).
+  static __device__ __forceinline__ float quad_of(uint32_t taddr) {
+    constexpr int R = DP % 32 == 0 ? 2 : 1;  // 16-column blocks per wait
     float q = 0.f;
 #pragma unroll
-    for (int c0 = 0; c0 < DP; c0 += 16) {
-      float v[16], u[16];
-      tmem_ld16x2(taddr + c0, taddr + DP + c0, v, u);
+    for (int c0 = 0; c0 < DP; c0 += 16 * R) {
+      uint32_t v[R][16], u[R][16];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (c0 + k < DP) {  // columns past 2 DP are not written by the MMAs
-          const float y = v[k] + u[k];
+      for (int r = 0; r < R; ++r) {
+        tmem_ld16(taddr + c0 + 16 * r, v[r]);
+        tmem_ld16(taddr + DP + c0 + 16 * r, u[r]);
+      }
+      tmem_wait();
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        tmem_use(v[r]);
+        tmem_use(u[r]);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float y = __uint_as_float(v[r][k]) + __uint_as_float(u[r][k]);
           q = fmaf(y, y, q);
         }
       }
     }
-    const int p = tid;
-    if (p >= meta.cnt) return;
-    if (MODE == ESTEP) {
-      const int32_t c = cidx[p];
-      float lr = NAN;
-      if (c >= 0) {
-        lr = __fadd_rn(__fmul_rn(q, meta.c1), meta.c0);
-        if ((int64_t)c == meta.n + g.koff) lr = -INFINITY;
-      }
-      g.logrho[meta.base + p] = lr;
-    } else {
-      float *pm = reinterpret_cast<float *>(sm + Smem::PM);
-      float *ps = pm + PQ;
-      const int qi = (int)meta.base + p;
-      // hardware log and exp: a few 1e-5 nats at most on the density
-      const float lp = meta.c0 - meta.c1 * __logf(1.f + q);
-      const float m = pm[qi];
-      if (lp > m) {
-        ps[qi] = ps[qi] * __expf(m - lp) + 1.f;
-        pm[qi] = lp;
-      } else {
-        ps[qi] += __expf(lp - m);
+    return q;
+  }
+
+  // log rho of the pairs of tile t (one warpgroup, lane = pair).
+  static __device__ __forceinline__ void epilogue_e(const Args &g, const unsigned char *sm, int t, uint32_t tacc,
+                                                    int w4, int lane) {
+    const Meta &m = meta_of(sm, t);
+    const int p = 32 * w4 + lane;
+    if (32 * w4 >= m.cnt) return;
+    const float q = quad_of(tacc + ((uint32_t)(w4 * 32) << 16));
+    if (p >= m.cnt) return;
+    const int32_t c = (reinterpret_cast<const int32_t *>(sm + Smem::CIDX) + (t % NS) * MT)[p];
+    float lr = NAN;
+    if (c >= 0) {
+      lr = __fadd_rn(__fmul_rn(q, m.c1), m.c0);
+      if ((int64_t)c == m.n + g.koff) lr = -INFINITY;
+    }
+    g.logrho[m.base + p] = lr;
+  }
+
+  // Student-t term of the kernel of tile t into the running (max, sum) of this
+  // thread's query; hardware log and exp: a few 1e-5 nats at most on the density.
+  static __device__ __forceinline__ void epilogue_p(const Meta &m, uint32_t tacc, int w4, float2 &run) {
+    if (32 * w4 >= m.cnt) return;
+    const float q = quad_of(tacc + ((uint32_t)(w4 * 32) << 16));
+    const float lp = m.c0 - m.c1 * __logf(1.f + q);
+    const bool up = lp > run.x;
+    const float e = __expf(up ? run.x - lp : lp - run.x);
+    if (lp != -INFINITY) {
+      run.y = up ? run.y * e + 1.f : run.y + e;
+      run.x = up ? lp : run.x;
+    }
+  }
+
+  // 16 columns c0 .. of an accumulator row, its two halves (c0 and 64 + c0) added.
+  static __device__ __forceinline__ void acc_row16(uint32_t taddr, int c0, bool empty, float (&x)[16]) {
+    uint32_t v[16], u[16];
+    if (!empty) {
+      tmem_ld16(taddr + c0, v);
+      tmem_ld16(taddr + 64 + c0, u);
+      tmem_wait();
+      tmem_use(v);
+      tmem_use(u);
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = empty ? 0.f : __uint_as_float(v[k]) + __uint_as_float(u[k]);
+  }
+
+  // S_n of the row whose last tile is t, by one warpgroup (rsum, badr: the row's
+  // sum of r and whether it has an invalid index).  Accumulator row i < 64
+  // holds (hh_ij, hl_ij) in columns (j, 64 + j), row 64 + i holds (lh_ij, ll_ij).
+  // Tiles: the warps of the lo rows put (lh + ll) into the group's shared copy,
+  // those of the hi rows add (hh + hl) and store row i of each tile, 256
+  // contiguous bytes per tile and eight lanes.  Dense rows: both halves go
+  // through the copy, so that a warp's stores are consecutive.  False when a
+  // wait ran out.
+  static __device__ bool epilogue_m(const Args &g, unsigned char *sm, uint64_t *bars, const Meta &m, uint32_t tacc,
+                                    int grp, int use, float rsum, bool badr, int w4, int lane) {
+    float *red = reinterpret_cast<float *>(sm + Smem::BST + (uint32_t)grp * Smem::B_BYTES);
+    const bool empty = (m.cnt == 0) && (m.flags & 1);
+    const bool bad = badr || (m.flags & 4) != 0;
+    const int half = w4 >> 1, ib = w4 & 1, i = 32 * ib + lane;  // accumulator row 64 half + i
+    const uint32_t taddr = tacc + ((uint32_t)(w4 * 32) << 16);
+    const int D = g.D;
+    const int64_t n = m.n;
+    constexpr int NCB = (DP + 15) / 16;
+    const bool through = half == 1 || !g.SPo;  // this warp writes the copy
+    if (through) {
+      // the group's last reads of the copy
+      if (use > 0 && !mbar_wait(bars + Bars::EFREE + grp, (uint32_t)((use - 1) & 1))) return false;
+#pragma unroll
+      for (int cb = 0; cb < NCB; ++cb) {
+        // rows 32 ib .. + 31 of the lower triangle
+        if (32 * ib >= DP || cb >= 2 * (ib + 1)) continue;
+        float x[16];
+        acc_row16(taddr, 16 * cb, empty, x);
+        if (i < DP) {
+#pragma unroll
+          for (int k = 0; k < 16; k += 4)
+            *reinterpret_cast<float4 *>(red + (half * DP + i) * Smem::RSTR + 16 * cb + k) =
+                make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+        }
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars + Bars::EFULL + grp);
+    if (w4 == 0 && lane == 0) g.nu_out[n] = bad ? NAN : g.nu0 + rsum;
+    const float *Uh = red, *Vl = red + DP * Smem::RSTR;
+    if (g.SPo) {
+      if (half == 0) {
+        if (!mbar_wait(bars + Bars::EFULL + grp, (uint32_t)(use & 1))) return false;
+        const int I = i >> 3;
+        float *dst = g.SPo + n * (int64_t)(g.ntile * 128) + (I * (I + 1) / 2) * 128 + (i & 7) * 8;
+#pragma unroll
+        for (int cb = 0; cb < NCB; ++cb) {
+          if (32 * ib >= DP || cb >= 2 * (ib + 1)) continue;
+          float x[16];
+          acc_row16(taddr, 16 * cb, empty, x);
+          if (i < DP) {
+#pragma unroll
+            for (int k = 0; k < 16; k += 4) {
+              const int j = 16 * cb + k, J = j >> 3;
+              const float4 a = *reinterpret_cast<const float4 *>(Vl + i * Smem::RSTR + j);
+              float4 v;
+              v.x = (i < D && j <= i) ? a.x + x[k] : 0.f;
+              v.y = (i < D && j + 1 <= i) ? a.y + x[k + 1] : 0.f;
+              v.z = (i < D && j + 2 <= i) ? a.z + x[k + 2] : 0.f;
+              v.w = (i < D && j + 3 <= i) ? a.w + x[k + 3] : 0.f;
+              if (bad) v = make_float4(NAN, NAN, NAN, NAN);
+              if (I < g.nt && J <= I) *reinterpret_cast<float4 *>(dst + J * 128 + (j & 7)) = v;
+            }
+          }
+        }
+      }
+    } else {
+      if (!mbar_wait(bars + Bars::EFULL + grp, (uint32_t)(use & 1))) return false;
+      float *Sn = g.S + n * (int64_t)D * D;
+      for (int r = w4; r < D; r += 4)
+        for (int j = lane; j < (g.lower_only ? r + 1 : D); j += 32) {
+          const int a = r > j ? r : j, b = r > j ? j : r;  // symmetric: from the lower triangle
+          Sn[r * D + j] = bad ? NAN : Vl[a * Smem::RSTR + b] + Uh[a * Smem::RSTR + b];
+        }
+    }
+    fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars + Bars::EFREE + grp);
+    return true;
   }
 };
 
-// Warps 0-7 convert and run the epilogue; warp 8 writes the tile metadata up
-// to NS - 2 tiles ahead; warps 9 .. 8 + NGW gather the pair rows (a share of
-// each tile's rows each; the first also the kernel centres and W cores) one
-// tile ahead; the last warp issues the MMAs of each converted tile.
-// Named barriers 1 and 2 count the NTHR consumer threads exactly.
-constexpr int WARP_META = NTHR / 32, WARP_GATHER = WARP_META + 1, WARP_MMA = WARP_GATHER + NGW;
-constexpr int NWARPS = WARP_MMA + 1;
-constexpr int NTHR_ALL = NWARPS * 32;
-
 template <int MODE, int DP>
-__global__ void __launch_bounds__(NTHR_ALL, 1) tc_kernel(Args g) {
+__global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) tc_kernel(Args g) {
   using K = Kern<MODE, DP>;
-  using Smem = SmemL<MODE>;
+  using Smem = Cfg<MODE, DP>;
+  constexpr int NA = Smem::NA, NCW = Smem::NCW, NEW = Smem::NEW, NGRP = Smem::NGRP;
+  constexpr int WARP_EPI = NCW, WARP_PLAN = NCW + NEW, WARP_MMA = WARP_PLAN + 1, WARP_COPY = WARP_PLAN + 2;
+  static_assert(NCW % 4 == 0 && NEW % 4 == 0, "a warp reads the TMEM lanes of its index mod 4");
+  constexpr int WARP_IDX = WARP_COPY + (MODE == MSTEP ? 0 : NCOPY);
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm + Smem::BAR);
+  uint64_t *pfull = bars + Bars::PFULL, *pempty = bars + Bars::PEMPTY;
   uint64_t *mfull = bars + Bars::MFULL, *mempty = bars + Bars::MEMPTY;
-  uint64_t *rfull = bars + Bars::RFULL, *rempty = bars + Bars::REMPTY;
   uint64_t *bfull = bars + Bars::BFULL, *bempty = bars + Bars::BEMPTY;
   uint64_t *mma_done = bars + Bars::MMA, *conv = bars + Bars::CONV;
-  const Meta *metas = reinterpret_cast<const Meta *>(sm + Smem::META);
 
-  // zero the operand tile (cores past DP stay zero) and the B stages (cores above the block diagonal)
-  for (uint32_t o = tid * 16; o < Smem::RAW; o += NWARPS * 32 * 16)
+  // zero the A tiles (cores past D, rows past a tile's end) and the B stages
+  // (cores above the block diagonal)
+  for (uint32_t o = tid * 16; o < Smem::CIDX; o += Smem::THREADS * 16)
     *reinterpret_cast<uint4 *>(sm + o) = make_uint4(0, 0, 0, 0);
   if (MODE != MSTEP)
-    for (uint32_t o = tid * 16; o < 4 * Smem::B_BYTES; o += NWARPS * 32 * 16)
-      *reinterpret_cast<uint4 *>(sm + Smem::BST + o) = make_uint4(0, 0, 0, 0);
-  if (MODE == PRED) {
-    float *pm = reinterpret_cast<float *>(sm + Smem::PM);
-    for (int i = tid; i < PQ; i += NWARPS * 32) {
-      pm[i] = -INFINITY;
-      pm[PQ + i] = 0.f;
-    }
-  }
-  if (warp == 0) tmem_alloc(&s_tmem, 2 * K::ACC_COLS);
+    for (int x = tid; x < 2 * g.ntile; x += Smem::THREADS)
+      reinterpret_cast<uint32_t *>(sm + Smem::TAB)[x] = K::core_offset(x, g.nt);
+  if (warp == 0) tmem_alloc(&s_tmem, 2 * Smem::ACC);
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) {
       mbar_init(mfull + i, 32);
-      mbar_init(mempty + i, 1);
+      mbar_init(mempty + i, NCW + NEW);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(rfull + i, 32 * NGW + 1);
-      mbar_init(rempty + i, 1);
-      mbar_init(bfull + i, 1);
+      mbar_init(pfull + i, 1);
+      mbar_init(pempty + i, NCW + NEW + (MODE == MSTEP ? 0 : NCOPY));
+      mbar_init(bfull + i, 32 * NCOPY);
       mbar_init(bempty + i, 1);
-    }
-    for (int i = 0; i < 2; ++i) {
       mbar_init(mma_done + i, 1);
-      mbar_init(conv + i, NTHR);
+      mbar_init(conv + i, NCW + (MODE == MSTEP ? 0 : 4));
+      mbar_init(bars + Bars::EFULL + i, 4);
+      mbar_init(bars + Bars::EFREE + i, 4);
+      mbar_init(bars + Bars::AFULL + i, 1);
+      mbar_init(bars + Bars::AFREE + i, 4);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -946,168 +920,285 @@ __global__ void __launch_bounds__(NTHR_ALL, 1) tc_kernel(Args g) {
   __syncthreads();
   fence_after();
   const uint32_t tmem = s_tmem;
+  const auto failed = [&]() {
+    if (lane == 0) atomicExch(g.err, 1);
+  };
+  // tile t planned; planned and its indices written; a warp done with tile t's plan
+  const auto planned = [&](int t) { return mbar_wait(pfull + ((t >> 5) & 1), (uint32_t)((t >> 6) & 1)); };
+  const auto ready = [&](int t) {
+    return MODE == PRED ? planned(t) : mbar_wait(mfull + t % NS, (uint32_t)((t / NS) & 1));
+  };
+  const auto unplan = [&](int t) {
+    if ((t & 31) == 31) mbar_arrive(pempty + ((t >> 5) & 1));
+  };
+  // predictive density: running (max, sum) of this thread's query in each query tile
+  float2 run0 = make_float2(-INFINITY, 0.f), run1 = run0;
 
   if (warp == WARP_MMA) {
     // ----------------------------------------------------------- MMA warp
-    int row_acc = 0;   // M-step: accumulator of the current row
-    int last = -1;     // last tile whose MMAs were issued
-
-    for (int t = 0;; ++t) {
-      const int ms = t % NS, s = t & 1;
-      if (!mbar_wait(mfull + ms, (uint32_t)((t / NS) & 1))) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
+    // No wait on the plan but the first: the converters have seen the plan of
+    // tile t + 1 before they arrive for tile t.
+    int last = -1;  // last tile whose MMAs were issued
+    bool ok = planned(0);
+    for (int t = 0; ok; ++t) {
+      const int s = t & 1;
+      const Meta &meta = K::meta_of(sm, t);
+      const int cnt = __shfl_sync(0xffffffffu, meta.cnt, 0), flags = __shfl_sync(0xffffffffu, meta.flags, 0);
+      const int row = __shfl_sync(0xffffffffu, meta.row, 0);
+      if (__shfl_sync(0xffffffffu, (int)(meta.n < 0), 0)) break;
+      if (flags & 1) {
+        if (MODE != MSTEP) ok = mbar_wait(bfull + (row & 1), (uint32_t)((row >> 1) & 1));
+        // the accumulator of row - 2 read
+        else if (row >= 2) ok = mbar_wait(bars + Bars::AFREE + (row & 1), (uint32_t)((row / 2 - 1) & 1));
       }
-      const Meta &meta = metas[ms];
-      if (meta.n < 0) break;
-      if (MODE != MSTEP && (meta.flags & 1) && !mbar_wait(bfull + meta.bs, (uint32_t)meta.bph)) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
-      }
-      if (!mbar_wait(conv + s, (uint32_t)((t / 2) & 1))) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
-      }
-      fence_after();
-      uint32_t acc_sel = (uint32_t)s;
-      if (MODE == MSTEP) {
-        if (meta.flags & 1) row_acc ^= 1;
-        acc_sel = (uint32_t)row_acc;
-      }
-      if (lane == 0) {
-        if (!Smem::DUAL) mbar_arrive(rempty + s);  // every converter has read raw stage s
-        K::issue_mma(g, sm, meta, tmem, acc_sel, s, mma_done + s);
-        if (Smem::DUAL) commit(rempty + s);  // A tile s free once its MMAs are done
-        if (MODE != MSTEP && (meta.flags & 2)) commit(bempty + meta.bs);
-      }
-      __syncwarp();
-      last = t;
-    }
-    // none of this warp's MMAs stays in flight (bounded wait)
-    if (last >= 0) mbar_wait(mma_done + (last & 1), (uint32_t)((last / 2) & 1));
-  } else if (warp == WARP_META) {
-    // ---------------------------------------------------- metadata warp
-    typename K::Prod P{};
-    P.n = -1;
-    typename K::Plan cur = K::plan_tile(g, P, lane), nxt{};
-    int32_t cc[4], nc[4];
-    float cw[4], nw[4];
-    K::load_tile(g, cur, lane, cc, cw);
-    for (int i = 0;; ++i) {
-      const int ms = i % NS;
-      if (cur.n >= 0) {
-        // the next tile's loads are in flight while this one is written
-        nxt = K::plan_tile(g, P, lane);
-        K::load_tile(g, nxt, lane, nc, nw);
-      }
-      if (i >= NS && !mbar_wait(mempty + ms, (uint32_t)((i / NS - 1) & 1))) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
-      }
-      K::write_tile(g, P, cur, cc, cw, sm, mfull + ms, ms, lane);
-      if (cur.n < 0) break;
-      cur = nxt;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cc[k] = nc[k];
-        cw[k] = nw[k];
-      }
-    }
-  } else if (warp >= WARP_GATHER && warp < WARP_GATHER + NGW) {
-    // ----------------------------------------------------- gather warps
-    const int gw = warp - WARP_GATHER;
-    int issued = 0;        // tiles whose copies this warp issued
-    int wlast0 = -1, wlast1 = -1;  // parity of the last W copy into B stage 0 / 1
-    bool first_tile = true;
-    for (int i = 0;; ++i) {
-      const int ms = i % NS, s = i & 1;
-      if (!mbar_wait(mfull + ms, (uint32_t)((i / NS) & 1))) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
-      }
-      const Meta &meta = metas[ms];
-      if (meta.n < 0) break;
-      if (i >= 2 && !mbar_wait(rempty + s, (uint32_t)((i / 2 - 1) & 1))) {
-        if (lane == 0) atomicExch(g.err, 1);
-        break;
-      }
-      if (gw == 0 && MODE != MSTEP && (meta.flags & 1)) {
-        if ((meta.flags & 8) && !mbar_wait(bempty + meta.bs, (uint32_t)(meta.bph ^ 1))) {
-          if (lane == 0) atomicExch(g.err, 1);
-          break;
-        }
-        K::copy_w(g, sm, meta, bfull + meta.bs, lane);
-        if (meta.bs) wlast1 = meta.bph;
-        else wlast0 = meta.bph;
-      }
-      K::gather(g, sm, meta, s, ms, rfull + s, g.stall && first_tile, gw, lane);
-      first_tile = false;
-      issued = i + 1;
-    }
-    // nothing of this warp's stays in flight: its row copies, then (bounded)
-    // the last phases of the stages it filled
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    for (int i = issued - 2; i < issued; ++i)
-      if (i >= 0) mbar_wait(rfull + (i & 1), (uint32_t)((i / 2) & 1));
-    if (wlast0 >= 0) mbar_wait(bfull, (uint32_t)wlast0);
-    if (wlast1 >= 0) mbar_wait(bfull + 1, (uint32_t)wlast1);
-  } else if (warp < WARP_META) {
-    // -------------------------------------------------- consumer warps
-    bool ok = true, epi_ok = true;
-    int t = 0;
-    int row_acc = 0;  // M-step: accumulator of the current row
-    int prev_acc = 0;
-    for (;; ++t) {
-      const int ms = t % NS, s = t & 1;
-      bool w = mbar_wait(mfull + ms, (uint32_t)((t / NS) & 1));
-      const Meta &meta = metas[ms];
-      const bool stop = w && meta.n < 0;
-      if (w && !stop) w = mbar_wait(rfull + s, (uint32_t)((t / 2) & 1));
-      // M-step: one A tile, rewritten only after the last tile's MMAs
-      if (!Smem::DUAL && t > 0) w = mbar_wait(mma_done + ((t - 1) & 1), (uint32_t)(((t - 1) / 2) & 1)) && w;
-      ok = bar_and(2, NTHR, w && epi_ok);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(conv + s, (uint32_t)((t / 2) & 1)));
       if (!ok) break;
       fence_after();
-      // tile t - 2's epilogue ran in the last iteration: its slot is free
-      if (tid == 0 && t >= 2) mbar_arrive(mempty + (t - 2) % NS);
-      uint32_t acc_sel = (uint32_t)s;
-      if (!stop) {
-        if (MODE == MSTEP) {
-          if (meta.flags & 1) row_acc ^= 1;
-          acc_sel = (uint32_t)row_acc;
-        }
-        K::convert(g, sm, s, ms, tid);
-        fence_async_smem();  // the tile is read by the MMAs (async proxy)
-        mbar_arrive(conv + s);
-      }
-      if (t > 0) {
-        // two A tiles: the previous tile's MMAs may still run (waited per warp;
-        // a time-out skips the epilogue and ends the loop at the next barrier)
-        if (Smem::DUAL)
-          epi_ok = __all_sync(0xffffffffu, mbar_wait(mma_done + ((t - 1) & 1), (uint32_t)(((t - 1) / 2) & 1)));
-        if (epi_ok) {
-          fence_after();
-          K::epilogue(g, sm, (t - 1) % NS, tmem, (uint32_t)prev_acc, tid);
-          fence_before();
-        }
-      }
-      prev_acc = (int)acc_sel;
-      if (stop) break;
+      K::issue_mma(g, sm, cnt, flags & 1, row, tmem, (MODE == MSTEP ? row : t) & 1, t % NA, mma_done + s);
+      if (flags & 2) commit(MODE == MSTEP ? bars + Bars::AFULL + (row & 1) : bempty + (row & 1));
+      last = t;
     }
-    if ((!ok || !epi_ok) && tid == 0) atomicExch(g.err, 1);  // the MMA warp waits for its own MMAs
+    if (!ok) failed();
+    // none of this warp's MMAs stays in flight (bounded wait)
+    if (last >= 0) mbar_wait(mma_done + (last & 1), (uint32_t)((last / 2) & 1));
+  } else if (warp == WARP_PLAN) {
+    // ------------------------------------------------------ planner warp
+    typename K::Batch P{};
+    for (int h = 0;; ++h) {
+      if (h >= 2 && !mbar_wait(pempty + (h & 1), (uint32_t)((h / 2 - 1) & 1))) {
+        failed();
+        break;
+      }
+      const bool more = K::plan_half(g, P, sm, 32 * h, lane);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pfull + (h & 1));
+      if (!more) break;
+    }
+  } else if (MODE != PRED && warp >= WARP_IDX) {
+    // ------------------------------------------------------- index warps
+    // one takes every NIDX-th tile, its next tile's loads in flight while it
+    // writes one (two register sets in turn: moving one set to the other would
+    // wait for the newest loads)
+    const int iw = warp - WARP_IDX;
+    int32_t c[2][4];
+    float w[2][4];
+    bool more = planned(iw);
+    if (!more) failed();
+    // tiles past the stop marker are not planned: every tile before is checked
+    int seen = 0;
+    const auto load = [&](int t, int32_t (&cc)[4], float (&ww)[4]) {
+      for (; seen <= t; ++seen) {
+        if ((seen & 31) == 0 && !planned(seen)) {
+          failed();
+          return false;
+        }
+        if (K::meta_of(sm, seen).n < 0) {
+          // the marker's slot: whoever would wait for it is let through
+          return false;
+        }
+      }
+      K::load_tile(g, K::meta_of(sm, t), lane, cc, ww);
+      return true;
+    };
+    const auto put = [&](int t, const int32_t (&cc)[4], const float (&ww)[4]) {
+      if (t >= NS && !mbar_wait(mempty + t % NS, (uint32_t)((t / NS - 1) & 1))) {
+        failed();
+        return false;
+      }
+      K::write_tile(g, K::meta_of(sm, t), cc, ww, sm, mfull + t % NS, t % NS, lane);
+      return true;
+    };
+    bool have = more && load(iw, c[0], w[0]);
+    int t = iw;
+    for (; have; t += 2 * NIDX) {
+      const bool h1 = load(t + NIDX, c[1], w[1]);
+      if (!put(t, c[0], w[0])) break;
+      if (!h1) {
+        t += NIDX;
+        break;
+      }
+      have = load(t + 2 * NIDX, c[0], w[0]);
+      if (!put(t + NIDX, c[1], w[1])) break;
+    }
+    // the stop marker is one of the next tiles: arrive for it if it is this
+    // warp's (its plan entry says stop, no indices are read)
+    if (seen % NIDX == iw && K::meta_of(sm, seen).n < 0 &&
+        (seen < NS || mbar_wait(mempty + seen % NS, (uint32_t)((seen / NS - 1) & 1))))
+      mbar_arrive(mfull + seen % NS);
+  } else if (MODE != MSTEP && warp >= WARP_COPY) {
+    // ------------------------------------------------------- copy warps
+    const int cw = warp - WARP_COPY;
+    bool first = true;
+    for (int t = 0;; ++t) {
+      if (!planned(t)) {
+        failed();
+        break;
+      }
+      const Meta &meta = K::meta_of(sm, t);
+      if (meta.n < 0) break;
+      if (meta.flags & 1) {
+        const int row = meta.row, bs = row & 1;
+        if (row >= 2 && !mbar_wait(bempty + bs, (uint32_t)((row / 2 - 1) & 1))) {
+          failed();
+          break;
+        }
+        K::copy_w(g, sm, meta, cw, lane);
+        // the copies land before the arrival (the MMAs read the stage through
+        // the async proxy); the test hook's first stage expects 16 bytes no
+        // copy delivers
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fence_async_smem();
+        if (g.stall && first && cw == 0 && lane == 0) mbar_arrive_tx(bfull + bs, 16);
+        else mbar_arrive(bfull + bs);
+        first = false;
+      }
+      __syncwarp();
+      if (lane == 0) unplan(t);
+    }
+  } else if (warp < NCW) {
+    // ------------------------------------------------- converter warps
+    typename K::Rows R = {};
+    bool ok = ready(0);
+    // predictive density: the CTA's queries, two tiles of them
+    constexpr int NPQ = MODE == PRED ? Smem::NP : 1;
+    float4 y[2][NPQ];
+    const int64_t q0 = MODE == PRED ? (int64_t)(blockIdx.x % g.nqb) * QB : 0;
+    const int k = lane & (Smem::LPR - 1), rch = (g.D + 3) / 4;
     if (MODE == PRED) {
-      bar_sync(2, NTHR);
-      const float *pm = reinterpret_cast<const float *>(sm + Smem::PM);
-      for (int64_t i = tid; i < g.qn; i += NTHR) {
-        g.ws_m[(int64_t)blockIdx.x * g.Nq + g.q0 + i] = pm[i];
-        g.ws_s[(int64_t)blockIdx.x * g.Nq + g.q0 + i] = pm[PQ + i];
+#pragma unroll
+      for (int tl = 0; tl < 2; ++tl)
+#pragma unroll
+        for (int i = 0; i < NPQ; ++i) {
+          const int64_t q = q0 + tl * MT + (i * Smem::NCW + warp) * Smem::RW + lane / Smem::LPR;
+          if (k < rch && q < g.Nq) y[tl][i] = ldg_row(g.Y + q * g.ldy + 4 * k);
+        }
+    }
+    if (ok && K::meta_of(sm, 0).n >= 0) {
+      K::load_rows(g, sm, 0, warp, lane, R);
+    }
+    for (int t = 0; ok; ++t) {
+      const Meta &meta = K::meta_of(sm, t);
+      if (meta.n < 0) break;
+      ok = ready(t + 1);
+      // the A tile's last MMAs
+      if (ok && t >= NA) ok = mbar_wait(mma_done + ((t - NA) & 1), (uint32_t)(((t - NA) / 2) & 1));
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      unsigned char *tile = sm + Smem::TILE + (uint32_t)(t % NA) * Smem::TILE_BYTES;
+      if (MODE == PRED) {
+        // base / 128: which of the CTA's two query tiles
+        if (k < rch) {
+          const float4 c = R.c;
+          const int cnt = meta.cnt;
+          const uint4 mask = K::dim_masks(k, g.D);
+          if (meta.base == 0) {
+#pragma unroll
+            for (int i = 0; i < NPQ; ++i) {
+              const int p = (i * NCW + warp) * Smem::RW + lane / Smem::LPR;
+              if (p < cnt) K::store_row(tile, p, k, y[0][i], c, mask);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < NPQ; ++i) {
+              const int p = (i * NCW + warp) * Smem::RW + lane / Smem::LPR;
+              if (p < cnt) K::store_row(tile, p, k, y[1][i], c, mask);
+            }
+          }
+        }
+      } else {
+        K::convert(g, sm, tile, t, warp, lane, R);
+      }
+      fence_async_smem();  // the tile is read by the MMAs (async proxy)
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(conv + (t & 1));
+        if (MODE != PRED) mbar_arrive(mempty + t % NS);
+      }
+      if (K::meta_of(sm, t + 1).n >= 0) K::load_rows(g, sm, t + 1, warp, lane, R);
+      if (lane == 0) unplan(t);
+    }
+    if (!ok) failed();
+  } else if (warp < WARP_PLAN) {
+    // -------------------------------------------------- epilogue warps
+    const int grp = (warp - WARP_EPI) >> 2, w4 = warp & 3;
+    const int step = MODE == PRED && g.Nq - (int64_t)(blockIdx.x % g.nqb) * QB > MT ? 2 : 1;  // query tiles
+    int use = 0;        // M-step: rows this warpgroup has finished
+    float rsum = 0.f;   // M-step: sum of r over the row so far
+    bool bad = false, ok = true;
+    // the first two tiles have no earlier accumulator to wait for
+    if (MODE != MSTEP && grp == 0 && lane < 2) mbar_arrive(conv + lane);
+    for (int t = 0;; ++t) {
+      ok = __all_sync(0xffffffffu, ready(t));
+      if (!ok) break;
+      const Meta &meta = K::meta_of(sm, t);
+      if (meta.n < 0) break;
+      const int flags = meta.flags, row = meta.row;
+      if (MODE == MSTEP) {
+        const float2 rs = reinterpret_cast<const float2 *>(sm + Smem::RS)[t % NS];
+        if (flags & 1) {
+          rsum = 0.f;
+          bad = false;
+        }
+        rsum += rs.x;
+        bad = bad || __float_as_uint(rs.y) != 0u;
+      }
+      const int acc = MODE == MSTEP ? row : t;  // uses of the accumulators in turn
+      if ((MODE != MSTEP || (flags & 2)) && acc % NGRP == grp) {
+        ok = __all_sync(0xffffffffu, mbar_wait((MODE == MSTEP ? bars + Bars::AFULL : mma_done) + (acc & 1),
+                                               (uint32_t)((acc / 2) & 1)));
+        if (!ok) break;
+        fence_after();
+        const uint32_t tacc = tmem + (uint32_t)(acc & 1) * Smem::ACC;
+        if (MODE == ESTEP) {
+          K::epilogue_e(g, sm, t, tacc, w4, lane);
+        } else if (MODE == PRED) {
+          if (step == 1 || (t & 1) == 0) K::epilogue_p(meta, tacc, w4, run0);
+          else K::epilogue_p(meta, tacc, w4, run1);
+        } else {
+          ok = __all_sync(0xffffffffu, K::epilogue_m(g, sm, bars, meta, tacc, grp, use, rsum, bad, w4, lane));
+          if (!ok) break;
+          ++use;
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive((MODE == MSTEP ? bars + Bars::AFREE : conv) + (acc & 1));
+      }
+      __syncwarp();
+      if (lane == 0) {
+        if (MODE != PRED) mbar_arrive(mempty + t % NS);
+        unplan(t);
       }
     }
+    if (!ok) failed();
   }
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == 0) tmem_dealloc(tmem, 2 * K::ACC_COLS);
+  if (MODE == PRED) {
+    // each epilogue warpgroup's partials of the query tiles it met
+    float2 *part = reinterpret_cast<float2 *>(sm + Smem::TILE);  // [NGRP][2][128], the A tiles are done
+    if (warp >= WARP_EPI && warp < WARP_PLAN) {
+      const int e = ((warp - WARP_EPI) >> 2) * QB + (warp & 3) * 32 + lane;
+      part[e] = run0;
+      part[e + MT] = run1;
+    }
+    __syncthreads();
+    const int64_t q0 = (int64_t)(blockIdx.x % g.nqb) * QB;
+    for (int e = tid; e < QB && q0 + e < g.Nq; e += Smem::THREADS) {
+      float m = -INFINITY, ssum = 0.f;
+#pragma unroll
+      for (int gr = 0; gr < NGRP; ++gr) m = fmaxf(m, part[gr * QB + e].x);
+#pragma unroll
+      for (int gr = 0; gr < NGRP; ++gr) {
+        const float2 a = part[gr * QB + e];
+        if (a.x != -INFINITY) ssum += a.y * __expf(a.x - m);
+      }
+      const int64_t o = (int64_t)(blockIdx.x / g.nqb) * g.Nq + q0 + e;
+      g.ws_m[o] = m;
+      g.ws_s[o] = ssum;
+    }
+  }
+  if (warp == 0) tmem_dealloc(tmem, 2 * Smem::ACC);
 }
 
 // W_triu (dense, upper) -> W cores: element X[i][j] = W_triu[j][i] (i >= j) of
@@ -1204,11 +1295,11 @@ int sm_count() {
   return sms;
 }
 
-// One persistent CTA per SM (the shared memory of the pipeline allows one).
+// Persistent CTAs, as many as are resident at once.
 template <int MODE, int DP>
 int launch_rows(const char *what, tc::Args g, int64_t rows, void *stream) {
   auto kern = tc::tc_kernel<MODE, DP>;
-  const size_t smem = tc::SmemL<MODE>::bytes;
+  const size_t smem = tc::Cfg<MODE, DP>::bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     set_error("%s: %s", what, cudaGetErrorString(e));
@@ -1222,10 +1313,14 @@ int launch_rows(const char *what, tc::Args g, int64_t rows, void *stream) {
       return LAKDE_ECUDA;
     }
   }
-  int64_t grid = sm_count();
+  int64_t grid = (int64_t)sm_count() * tc::Cfg<MODE, DP>::CTAS;
   if (grid > rows) grid = rows;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, tc::NTHR_ALL, smem, as_stream(stream)>>>(g);
+  // eight or more claims per CTA (the tail and small row counts balance), at
+  // most a row per lane of the metadata warp
+  const int64_t batch = rows / (8 * grid);
+  g.batch = (int)(batch < 1 ? 1 : batch > 32 ? 32 : batch);
+  kern<<<(unsigned)grid, tc::Cfg<MODE, DP>::THREADS, smem, as_stream(stream)>>>(g);
   return check_launch(what);
 }
 
@@ -1397,15 +1492,21 @@ extern "C" int lakde_mstep_tc_tiled(int dtype, int64_t N, int64_t D, int64_t npt
                          nullptr, 0, SP, nu, queue, err, stream);
 }
 
-static int64_t pred_tc_chunks(int64_t N) {
-  int64_t nchunks = sm_count();  // one CTA per SM
+// Chunks of kernels: the blocks of 256 queries times the chunks make up to
+// four full waves of the resident CTAs (a CTA keeps its queries for its whole
+// chunk, so longer chunks only save its set-up).
+static int64_t pred_tc_chunks(int64_t N, int64_t Nq, int64_t D) {
+  const int64_t nqb = (Nq + tc::QB - 1) / tc::QB;
+  const int64_t resident = (int64_t)sm_count() * (D <= 32 ? 2 : 1);
+  int64_t nchunks = 4 * resident / nqb;
+  if (nqb * N < 64 * resident * 4) nchunks = resident / nqb;  // little work: one wave
   if (nchunks > N) nchunks = N;
   return nchunks < 1 ? 1 : nchunks;
 }
 
 extern "C" size_t lakde_log_pred_density_tc_workspace(int64_t N, int64_t Nq, int64_t D) {
   if (N <= 0 || Nq <= 0 || D < 1 || D > 64) return 0;
-  return (size_t)(2 * pred_tc_chunks(N) * Nq) * sizeof(float);
+  return (size_t)(2 * pred_tc_chunks(N, Nq, D) * Nq) * sizeof(float);
 }
 
 extern "C" int lakde_log_pred_density_tc(int dtype, int64_t N, int64_t Nq, int64_t D, const void *X, int64_t ldx,
@@ -1437,7 +1538,7 @@ extern "C" int lakde_log_pred_density_tc(int dtype, int64_t N, int64_t Nq, int64
     return LAKDE_EINVAL;
   }
   if (int st = bind_device("log_pred_density_tc", {out, X, W_cores, nu, log_coeff, Y, workspace, err})) return st;
-  const int64_t nchunks = pred_tc_chunks(N);
+  const int64_t nchunks = pred_tc_chunks(N, Nq, D);
   tc::Args g{};
   g.X = static_cast<const float *>(X);
   g.ldx = ldx;
@@ -1450,32 +1551,32 @@ extern "C" int lakde_log_pred_density_tc(int dtype, int64_t N, int64_t Nq, int64
   g.ws_s = g.ws_m + nchunks * Nq;
   g.N = N;
   g.Nq = Nq;
-  g.npts = Nq;
+  g.npts = N;
+  g.nqb = (Nq + tc::QB - 1) / tc::QB;
   g.chunk = (N + nchunks - 1) / nchunks;
   g.D = (int)D;
   g.nt = tile_blocks(D);
   g.ntile = tile_total(D);
   g.err = err;
-  const int64_t grid = (N + g.chunk - 1) / g.chunk;
+  const int64_t used = (N + g.chunk - 1) / g.chunk;  // chunks with kernels
+  if (used * g.nqb > 0x7fffffffLL) {
+    set_error("log_pred_density_tc: problem too large");
+    return LAKDE_EUNSUPPORTED;
+  }
   int st = dispatch_tc(D, [&](auto dp) {
     constexpr int DP = decltype(dp)::value;
     auto kern = tc::tc_kernel<tc::PRED, DP>;
-    const size_t smem = tc::SmemL<tc::PRED>::bytes;
+    const size_t smem = tc::Cfg<tc::PRED, DP>::bytes;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
       set_error("log_pred_density_tc: %s", cudaGetErrorString(e));
       return (int)LAKDE_ECUDA;
     }
-    for (int64_t q0 = 0; q0 < Nq; q0 += tc::PQ) {
-      g.q0 = q0;
-      g.qn = (Nq - q0) < tc::PQ ? (Nq - q0) : tc::PQ;
-      kern<<<(unsigned)grid, tc::NTHR_ALL, smem, as_stream(stream)>>>(g);
-      if (int s2 = check_launch("log_pred_density_tc")) return s2;
-    }
-    return (int)LAKDE_OK;
+    kern<<<(unsigned)(used * g.nqb), tc::Cfg<tc::PRED, DP>::THREADS, smem, as_stream(stream)>>>(g);
+    return check_launch("log_pred_density_tc");
   });
   if (st) return st;
   sweep::fold_kernel<float><<<(unsigned)((Nq + 31) / 32), 256, 0, as_stream(stream)>>>(
-      g.ws_m, g.ws_s, static_cast<float *>(out), Nq, grid, (float)log((double)N));
+      g.ws_m, g.ws_s, static_cast<float *>(out), Nq, used, (float)log((double)N));
   return check_launch("log_pred_density_tc_fold");
 }
