@@ -142,6 +142,197 @@ __global__ void __launch_bounds__(kKnnThreadsLarge) knn_select_kernel(const doub
   }
 }
 
+// ------------------------------------------------- a warp per row (small k)
+// The same selection with one warp per row and no block barrier: the warp
+// streams 256 values at a time (four 16-byte loads per lane in flight) and
+// appends those below its threshold by ballot.  When the next 256 could overflow
+// its buffer it cuts it by bisection on the value to between kc and 3/2 kc
+// entries (about ten counting passes over 512 entries, 1k instructions; a
+// bitonic sort of them takes 7k, and four warps per row with a quarter each, so
+// four times the sorts, were slower than one), and sorts only what is left at
+// the end.
+constexpr int kWarpRows = 8;    // warps (rows) per block
+constexpr int kWarpStep = 256;  // values a warp scans between buffer checks
+
+__device__ __forceinline__ void warp_bitonic_sort(double *key, int32_t *idx, int n, int lane) {
+  for (int size = 2; size <= n; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      __syncwarp();
+      for (int t = lane; t < n / 2; t += 32) {
+        const int lo = 2 * t - (t & (stride - 1));
+        const int hi = lo + stride;
+        const bool up = (lo & size) == 0;
+        const double ka = key[lo], kb = key[hi];
+        const int32_t ia = idx[lo], ib = idx[hi];
+        const bool a_gt_b = ka > kb || (ka == kb && ia > ib);
+        if (a_gt_b == up) {
+          key[lo] = kb;
+          key[hi] = ka;
+          idx[lo] = ib;
+          idx[hi] = ia;
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
+template <typename I, typename O, int CAP>
+__global__ void __launch_bounds__(32 * kWarpRows) knn_select_warp_kernel(const double *__restrict__ dist, int64_t nb,
+                                                                         int64_t N, int64_t row0,
+                                                                         const double *__restrict__ X, int D,
+                                                                         int include_self, int k, int kc,
+                                                                         I *__restrict__ out_idx,
+                                                                         O *__restrict__ out_dist) {
+  extern __shared__ double knn_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  double *key = knn_smem + warp * CAP;
+  int32_t *idx = reinterpret_cast<int32_t *>(knn_smem + kWarpRows * CAP) + warp * CAP;
+  const int64_t r = (int64_t)blockIdx.x * kWarpRows + warp;
+  if (r >= nb) return;
+  const int64_t self = row0 + r;
+  const double *drow = dist + r * N;
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  int cnt = 0;
+  double thr = inf;  // later values at or above it are not among the kc smallest
+
+  // sorts the cnt entries (padded with +inf) and keeps the kc smallest
+  const auto sort_cut = [&]() {
+    int n = 32;
+    while (n < cnt) n <<= 1;
+    for (int t = cnt + lane; t < n; t += 32) {
+      key[t] = inf;
+      idx[t] = 0x7fffffff;
+    }
+    warp_bitonic_sort(key, idx, n, lane);
+    if (cnt >= kc) {
+      cnt = kc;
+      thr = key[kc - 1];
+    }
+  };
+  // keeps the entries up to a pivot with kc to 3/2 kc of them: every later value
+  // that is not below the pivot has kc predecessors.  Sorts when no such pivot is
+  // found in 40 halvings (many equal values).
+  const auto cut = [&]() {
+    if (cnt < kc) return;
+    __syncwarp();
+    double lo = inf, hi = -inf;
+    for (int t = lane; t < cnt; t += 32) {
+      lo = fmin(lo, key[t]);
+      hi = fmax(hi, key[t]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    const int most = kc + kc / 2;
+    int c = cnt;
+    double pivot = hi;
+    for (int it = 0; it < 40 && c > most; ++it) {
+      const double mid = lo + 0.5 * (hi - lo);
+      int m = 0;
+      for (int t = lane; t < cnt; t += 32) m += key[t] <= mid;
+      m = __reduce_add_sync(0xffffffffu, m);
+      if (m < kc) {
+        lo = mid;
+      } else {
+        hi = pivot = mid;
+        c = m;
+      }
+    }
+    if (c > most) {
+      sort_cut();
+      return;
+    }
+    // entries up to the pivot move forward, in order; a batch is read before
+    // any of it is overwritten
+    int kept = 0;
+    for (int t0 = 0; t0 < cnt; t0 += 32) {
+      const int t = t0 + lane;
+      const double v = t < cnt ? key[t] : inf;
+      const int32_t i = t < cnt ? idx[t] : 0;
+      const bool keep = t < cnt && v <= pivot;
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int p = kept + __popc(m & below);
+        key[p] = v;
+        idx[p] = i;
+      }
+      kept += __popc(m);
+      __syncwarp();
+    }
+    cnt = kept;
+    thr = pivot;
+  };
+
+  // 1. threshold scan
+  const bool vec = (reinterpret_cast<uintptr_t>(drow) & 15u) == 0;
+  for (int64_t base = 0; base < N; base += kWarpStep) {
+    if (cnt + kWarpStep > CAP) cut();
+    double v[kWarpStep / 32];
+    // value e of this lane is column base + 64 (e / 2) + 2 lane + e % 2
+    if (vec && base + kWarpStep <= N) {
+#pragma unroll
+      for (int e = 0; e < kWarpStep / 32; e += 2) {
+        const double2 d2 = __ldcs(reinterpret_cast<const double2 *>(drow + base + 32 * e + 2 * lane));
+        v[e] = d2.x;
+        v[e + 1] = d2.y;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < kWarpStep / 32; ++e) {
+        const int64_t j = base + 64 * (e / 2) + 2 * lane + (e & 1);
+        v[e] = j < N ? drow[j] : inf;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kWarpStep / 32; ++e) {
+      const int64_t j = base + 64 * (e / 2) + 2 * lane + (e & 1);
+      const bool in = v[e] < thr && (include_self || j != self);  // false for NaN
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (m == 0) continue;
+      if (in) {
+        const int p = cnt + __popc(m & below);
+        key[p] = v[e];
+        idx[p] = (int32_t)j;
+      }
+      cnt += __popc(m);
+    }
+  }
+  cut();
+  sort_cut();
+
+  // 2. exact re-ranking of the kc candidates
+  int n2 = 32;
+  while (n2 < kc) n2 <<= 1;
+  const double *xr = X + self * D;
+  for (int t = lane; t < n2; t += 32) {
+    double e = inf;
+    int32_t c = 0x7fffffff;
+    if (t < cnt) {
+      c = idx[t];
+      const double *xc = X + (int64_t)c * D;
+      double s = 0.0;
+#pragma unroll 4
+      for (int d = 0; d < D; ++d) {
+        const double df = xc[d] - xr[d];
+        s = fma(df, df, s);
+      }
+      e = s;
+    }
+    key[t] = e;
+    idx[t] = c;
+  }
+  warp_bitonic_sort(key, idx, n2, lane);
+  for (int t = lane; t < k; t += 32) {
+    const int32_t c = idx[t];
+    out_idx[r * k + t] = (I)(c == 0x7fffffff ? -1 : c);
+    if (out_dist) out_dist[r * k + t] = (O)sqrt(key[t]);
+  }
+}
+
 }  // namespace lakde
 
 using namespace lakde;
@@ -176,9 +367,29 @@ extern "C" int lakde_knn_select(const void *dist, int64_t nb, int64_t N, int64_t
   }
   if (int st = bind_device("knn_select", {dist, X, out_idx, out_dist})) return st;
   cudaStream_t s = as_stream(stream);
+  auto launch_warps = [&](auto ti, auto to, auto tc) {
+    using I = decltype(ti);
+    using O = decltype(to);
+    constexpr int CAP = decltype(tc)::value;
+    auto kern = knn_select_warp_kernel<I, O, CAP>;
+    constexpr size_t bytes = (size_t)kWarpRows * CAP * (sizeof(double) + sizeof(int32_t));
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      set_error("knn_select: cannot reserve %zu bytes of shared memory", bytes);
+      return (int)LAKDE_ECUDA;
+    }
+    kern<<<(unsigned)((nb + kWarpRows - 1) / kWarpRows), 32 * kWarpRows, bytes, s>>>(
+        static_cast<const double *>(dist), nb, N, row0, static_cast<const double *>(X), (int)D, include_self, (int)k,
+        (int)kc, static_cast<I *>(out_idx), static_cast<O *>(out_dist));
+    return check_launch("knn_select");
+  };
   auto launch = [&](auto ti, auto to) {
     using I = decltype(ti);
     using O = decltype(to);
+    // a warp per row while 3/2 of its candidates and a step fit its buffer: 6 KB
+    // up to 160 candidates (32 rows an SM in flight), 12 KB up to 500; beyond, a
+    // block per row, whose barriers cost less than a lone warp's sorts
+    if (kc <= 160) return launch_warps(ti, to, std::integral_constant<int, 512>{});
+    if (kc <= 500) return launch_warps(ti, to, std::integral_constant<int, 1024>{});
     auto kern = knn_select_kernel<I, O>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
       set_error("knn_select: cannot reserve %zu bytes of shared memory", smem);

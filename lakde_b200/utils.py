@@ -50,23 +50,28 @@ def batched_knn_cov(X, X_self, knn_graph, include_self=False, self_center=True):
 def compute_knn_graph(X, k, bsize=1024, return_dists=False, include_self=False, metric="l2", dtype=torch.int32):
     """k nearest neighbours of every row of X, nearest first (lakde/utils.py:77-116).
 
-    Per block of rows, one library GEMM gives the float64 squared distances
-    |a|^2 + |b|^2 - 2ab to all points; lakde_knn_select (kernels.knn_select)
-    keeps each row's k + 8 smallest in one pass, re-ranks them by exact
-    float64 differences and writes the k nearest, equal distances ordered by
-    index.
+    Per block of rows, one library GEMM gives the float64 squared distances to
+    all points less the row's own |a|^2, which does not change a row's order:
+    [-2a, 1] [b, |b|^2]^T = |b|^2 - 2ab, in one pass over the block;
+    lakde_knn_select (kernels.knn_select) keeps each row's k + 8 smallest in one
+    pass, re-ranks them by exact float64 differences and writes the k nearest,
+    equal distances ordered by index.
     """
     if metric.lower() != "l2":
         raise ValueError("only the l2 metric is supported")
     N = X.size(0)
     Xd = X.double().contiguous()
-    sq = (Xd * Xd).sum(1)
+    right = torch.cat((Xd, (Xd * Xd).sum(1, keepdim=True)), 1).T
+    left = torch.cat((-2.0 * Xd, Xd.new_ones(N, 1)), 1)
+    # at least 2 GB of distances a block (enough rows for the selection, a warp
+    # each, to fill the GPU), bsize rows when those are more
+    bsize = min(N, max(bsize, 2**28 // N))
+    d = Xd.new_empty(bsize, N)
     I = torch.empty(N, k, dtype=dtype, device=X.device)
     Dout = X.new_empty(N, k) if return_dists else None
     for i in range(0, N, bsize):
-        Xb = Xd[i : i + bsize]
-        d = torch.addmm(sq[None, :], Xb, Xd.T, alpha=-2.0).add_(sq[i : i + bsize, None])
-        kernels.knn_select(d, Xd, i, k, include_self=include_self, out_idx=I[i : i + bsize],
+        db = torch.mm(left[i : i + bsize], right, out=d[: N - i])
+        kernels.knn_select(db, Xd, i, k, include_self=include_self, out_idx=I[i : i + bsize],
                            out_dist=None if Dout is None else Dout[i : i + bsize])
     if return_dists:
         return Dout, I
