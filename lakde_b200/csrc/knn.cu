@@ -4,7 +4,7 @@
 // turns each row of the block into that point's k nearest neighbours, nearest
 // first, equal distances ordered by index:
 //
-//   1. one CTA per row streams the row once, keeping every value below a
+//   1. one CTA (small k: one warp) per row streams the row once, keeping every value below a
 //      running threshold in a shared-memory buffer; when the next chunk could
 //      overflow the buffer it is sorted (bitonic, by value then index) and cut
 //      to its kc = k + 8 smallest, whose largest becomes the threshold;
@@ -150,7 +150,9 @@ __global__ void __launch_bounds__(kKnnThreadsLarge) knn_select_kernel(const doub
 // entries (about ten counting passes over 512 entries, 1k instructions; a
 // bitonic sort of them takes 7k, and four warps per row with a quarter each, so
 // four times the sorts, were slower than one), and sorts only what is left at
-// the end.
+// the end.  Whole graph of 50,000 points at d = 21, k = 64: selection 24.4 -> 5.0
+// ms (one pass over the 20 GB of distances is 3.1), with the GEMM 49.0 -> 12.9;
+// 100,003 points at d = 63, k = 100: 169 -> 65 ms.
 constexpr int kWarpRows = 8;    // warps (rows) per block
 constexpr int kWarpStep = 256;  // values a warp scans between buffer checks
 
