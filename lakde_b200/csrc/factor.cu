@@ -186,7 +186,12 @@ struct DmmaCfg {
   // memory) and no L output: ~19 KB per warp at DP = 64, one warp per block,
   // 11 blocks per SM (registers capped to fit)
   static constexpr int WPB = LEAN ? 1 : 2;
-  static constexpr int BLOCKS_PER_SM = LEAN ? 11 : 1;
+  // up to DP = 32 the registers are capped at 128, so that 16 warps an SM hide the
+  // sweep's latencies instead of the 8 that 206 registers allow (60,000 matrices,
+  // tiled with trace: d = 21 0.380 -> 0.268 ms, d = 13 0.256 -> 0.164; a cap of 102
+  // spills: 0.308 and 0.179).  At 48 a cap of 168 gave 0.535 instead of 0.502 ms
+  // for 30,000 matrices, and at 64 shared memory holds eight matrices anyway
+  static constexpr int BLOCKS_PER_SM = LEAN ? 11 : DP <= 32 ? 8 : 1;
   // per warp: FP64 tiles, 1 / L_ii, then the lower triangle of a per-matrix
   // FP32 T_n (packed rows or tiles, in doubles rounded up to 16 bytes), which
   // doubles as the scratch tile of the L output (T_n is then not staged)
