@@ -2,88 +2,125 @@
 // FP64 (lakde/local_hierarchical_kde.py:293-297):
 //   out = sum_n w_n W_triu_n W_triu_n^T        (D x D, symmetric)
 // straight from the float32 (or float64) factors, without a float64 copy of
-// all of them.  Each CTA walks a contiguous chunk of kernels, stages W_triu_n
-// transposed in shared memory (column j of W as a row, zero below the
-// diagonal), and each thread accumulates one 4 x 4 block of the lower
-// triangle in FP64 registers: per column j two 16-byte loads of its block's
-// rows and two of its block's columns feed 16 FMAs.  The per-CTA partials are
-// summed in a fixed order by the final kernel, so the result does not depend
-// on scheduling.
+// all of them, on the FP64 tensor cores: each warp walks every (blocks x
+// warps)-th kernel with the lower 8 x 8 tiles of the sum in registers.  A step
+// takes four columns j of W_n: lane l holds W[8 I + l / 4][j + l % 4] of each row
+// block I, which is the A fragment of rows I (scaled by w_n) and, the product
+// being with W^T, the B fragment of columns I; the next eight columns' loads
+// are in flight under a block's products.  Rows below the diagonal block are
+// zero and not loaded.  The warps' sums are added in a fixed order, per block
+// and then over the blocks, so the result does not depend on scheduling.
+//
+// Bound by the FP64 tensor pipe: NT (NT + 1) (NT + 2) / 3 MMAs of 16 cycles per
+// kernel.  20,000 kernels at d = 43: 350 + 64 -> 89 + 5 us (scalar FMAs on 4 x 4
+// register blocks staged through shared memory, and one thread walking all
+// partials of an element, before).
 #include "common.cuh"
+#include "factor_dmma.cuh"
 
 namespace lakde {
 
-constexpr int kGramBlocks = 592;
-constexpr int kGramThreads = 160;  // >= the 136 lower 4 x 4 blocks at D = 64
+constexpr int kGramBlocks = 592;  // partials the workspace has room for
+constexpr int kGramWarps = 4;
 
-template <typename T>
-__global__ void __launch_bounds__(kGramThreads) gram_partial_kernel(const T *__restrict__ W, const T *__restrict__ w,
-                                                                   int64_t N, int D, int64_t chunk,
-                                                                   double *__restrict__ partials) {
-  extern __shared__ double sWt[];  // [DP][DP]: sWt[j * DP + i] = W[i][j] for j >= i, else 0
-  const int DP = (D + 3) & ~3, nb = DP / 4;
-  const int tri = D * (D + 1) / 2;
-  const int tid = threadIdx.x;
-  int bi = 0;
-  while ((bi + 1) * (bi + 2) / 2 <= tid) ++bi;
-  const int bk = tid - bi * (bi + 1) / 2;
-  const bool active = bi < nb;
-  double acc[4][4];
+template <typename T, int NT>
+__device__ __forceinline__ void gram_load(const T *__restrict__ Wn, int J, int D, int lane, T (&f)[NT][2]) {
+  const int r = lane >> 2, c = 8 * J + (lane & 3);
 #pragma unroll
-  for (int x = 0; x < 4; ++x)
+  for (int I = 0; I < NT; ++I) {
+    if (I > J) continue;
 #pragma unroll
-    for (int y = 0; y < 4; ++y) acc[x][y] = 0.0;
-  const int64_t n0 = (int64_t)blockIdx.x * chunk;
-  const int64_t n1 = (n0 + chunk < N) ? n0 + chunk : N;
-  for (int64_t n = n0; n < n1; ++n) {
-    const T *Wn = W + n * (int64_t)D * D;
-    __syncthreads();
-    // coalesced over the row-major W_triu_n, stored transposed
-    for (int e = tid; e < DP * DP; e += kGramThreads) {
-      const int i = e / DP, j = e % DP;
-      sWt[j * DP + i] = (i < D && j < D && j >= i) ? (double)Wn[i * D + j] : 0.0;
+    for (int s = 0; s < 2; ++s) {
+      const int i = 8 * I + r, j = c + 4 * s;
+      f[I][s] = (i <= j && j < D) ? Wn[(int64_t)i * D + j] : T(0);
     }
-    __syncthreads();
-    if (!active) continue;
-    const double wn = (double)w[n];
-    double t[4][4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) t[x][y] = 0.0;
-    // (W W^T)_ik = sum_j W_ij W_kj over j >= max(i, k) >= 4 bk
-    for (int j = 4 * bk; j < DP; ++j) {
-      const double *col = sWt + j * DP;
-      const double2 a01 = *reinterpret_cast<const double2 *>(col + 4 * bi);
-      const double2 a23 = *reinterpret_cast<const double2 *>(col + 4 * bi + 2);
-      const double2 b01 = *reinterpret_cast<const double2 *>(col + 4 * bk);
-      const double2 b23 = *reinterpret_cast<const double2 *>(col + 4 * bk + 2);
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y}, b[4] = {b01.x, b01.y, b23.x, b23.y};
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) t[x][y] = fma(a[x], b[y], t[x][y]);
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) acc[x][y] = fma(wn, t[x][y], acc[x][y]);
   }
-  if (!active) return;
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < 4; ++y) {
-      const int i = 4 * bi + x, k = 4 * bk + y;
-      if (i < D && k <= i) partials[(int64_t)blockIdx.x * tri + i * (i + 1) / 2 + k] = acc[x][y];
-    }
 }
 
-__global__ void gram_final_kernel(const double *__restrict__ partials, int nparts, int D, double *__restrict__ out) {
+template <typename T, int NT>
+__global__ void __launch_bounds__(32 * kGramWarps) gram_partial_kernel(const T *__restrict__ W, const T *__restrict__ w,
+                                                                      int64_t N, int D,
+                                                                      double *__restrict__ partials) {
+  constexpr int NTILE = NT * (NT + 1) / 2;
+  __shared__ double red[NTILE * 64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double acc[NTILE][2];
+#pragma unroll
+  for (int t = 0; t < NTILE; ++t) acc[t][0] = acc[t][1] = 0.0;
+  const int64_t stride = (int64_t)gridDim.x * kGramWarps, DD = (int64_t)D * D;
+  int64_t n = (int64_t)blockIdx.x * kGramWarps + warp;
+  T f[2][NT][2];
+  T wn = T(0);
+  if (n < N) {
+    gram_load<T, NT>(W + n * DD, 0, D, lane, f[0]);
+    wn = w[n];
+  }
+  while (n < N) {
+    const int64_t nn = n + stride;
+    const double wd = (double)wn;
+#pragma unroll
+    for (int J = 0; J < NT; ++J) {
+      // block J is in f[J % 2] (NT even: the next kernel's block 0 in f[0])
+      if (J + 1 < NT) {
+        gram_load<T, NT>(W + n * DD, J + 1, D, lane, f[(J + 1) & 1]);
+      } else if (NT % 2 == 0 && nn < N) {
+        gram_load<T, NT>(W + nn * DD, 0, D, lane, f[0]);
+        wn = w[nn];
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        double b[NT];
+#pragma unroll
+        for (int I = 0; I < NT; ++I)
+          if (I <= J) b[I] = (double)f[J & 1][I][s];
+#pragma unroll
+        for (int I = 0; I < NT; ++I) {
+          if (I > J) continue;
+          const double a = wd * b[I];
+#pragma unroll
+          for (int k = 0; k <= I; ++k) dmma::mma(acc[I * (I + 1) / 2 + k][0], acc[I * (I + 1) / 2 + k][1], a, b[k]);
+        }
+      }
+    }
+    if (NT % 2 == 1 && nn < N) {
+      gram_load<T, NT>(W + nn * DD, 0, D, lane, f[0]);
+      wn = w[nn];
+    }
+    n = nn;
+  }
+  // the warps' sums in turn
+  for (int v = 0; v < kGramWarps; ++v) {
+    if (warp == v) {
+#pragma unroll
+      for (int t = 0; t < NTILE; ++t) {
+        double *r = red + t * 64 + (lane >> 2) * 8 + 2 * (lane & 3);
+        r[0] = (v ? r[0] : 0.0) + acc[t][0];
+        r[1] = (v ? r[1] : 0.0) + acc[t][1];
+      }
+    }
+    __syncthreads();
+  }
   const int tri = D * (D + 1) / 2;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tri; e += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int p = 0; p < nparts; ++p) s += partials[(int64_t)p * tri + e];
+  for (int e = threadIdx.x; e < NTILE * 64; e += 32 * kGramWarps) {
+    int I = 0;
+    const int t = e >> 6;
+    while ((I + 1) * (I + 2) / 2 <= t) ++I;
+    const int i = 8 * I + ((e >> 3) & 7), k = 8 * (t - I * (I + 1) / 2) + (e & 7);
+    if (i < D && k <= i) partials[(int64_t)blockIdx.x * tri + i * (i + 1) / 2 + k] = red[e];
+  }
+}
+
+// One warp per element, its lanes over the partials (fixed order).
+__global__ void __launch_bounds__(256) gram_final_kernel(const double *__restrict__ partials, int nparts, int D,
+                                                         double *__restrict__ out) {
+  const int tri = D * (D + 1) / 2, lane = threadIdx.x & 31;
+  const int e = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (e >= tri) return;
+  double s = 0.0;
+#pragma unroll 4
+  for (int p = lane; p < nparts; p += 32) s += partials[(int64_t)p * tri + e];
+  s = warp_sum(s);
+  if (lane == 0) {
     int i = 0;
     while ((i + 1) * (i + 2) / 2 <= e) ++i;
     const int k = e - i * (i + 1) / 2;
@@ -120,13 +157,19 @@ extern "C" int lakde_weighted_gram(int dtype, int64_t N, int64_t D, const void *
   if (int st = bind_device("weighted_gram", {out, W_triu, w, workspace})) return st;
   return dispatch_float(dtype, [&](auto t0) {
     using T = decltype(t0);
-    const int64_t chunk = N > 0 ? (N + kGramBlocks - 1) / kGramBlocks : 1;
     double *part = static_cast<double *>(workspace);
-    const int DP = (int)((D + 3) & ~3);
-    gram_partial_kernel<T><<<kGramBlocks, kGramThreads, (size_t)DP * DP * sizeof(double), as_stream(stream)>>>(
-        static_cast<const T *>(W_triu), static_cast<const T *>(w), N, (int)D, chunk, part);
-    if (int st = check_launch("weighted_gram")) return st;
-    gram_final_kernel<<<8, 256, 0, as_stream(stream)>>>(part, kGramBlocks, (int)D, out);
-    return check_launch("weighted_gram_final");
+    return dispatch_dp(D, [&](auto dp) {
+      constexpr int NT = (decltype(dp)::value + 7) / 8;
+      // three blocks an SM (two at 64 dimensions: the sum's tiles in registers)
+      int64_t blocks = (N + kGramWarps - 1) / kGramWarps;
+      const int64_t most = 148 * (NT >= 8 ? 2 : 3);
+      blocks = blocks < 1 ? 1 : blocks > most ? most : blocks;
+      gram_partial_kernel<T, NT><<<(unsigned)blocks, 32 * kGramWarps, 0, as_stream(stream)>>>(
+          static_cast<const T *>(W_triu), static_cast<const T *>(w), N, (int)D, part);
+      if (int st = check_launch("weighted_gram")) return st;
+      const int tri = (int)(D * (D + 1) / 2);
+      gram_final_kernel<<<(unsigned)((tri + 7) / 8), 256, 0, as_stream(stream)>>>(part, (int)blocks, (int)D, out);
+      return check_launch("weighted_gram_final");
+    });
   });
 }
