@@ -66,19 +66,21 @@ __device__ __forceinline__ void load_row(const T *__restrict__ X, int64_t m, int
   const uintptr_t base = reinterpret_cast<uintptr_t>(X);
   // rows of 32 bytes (or 64) from a 32-byte aligned base: one 256-bit load
   // per 32 bytes, so a warp's gather of scattered rows touches each row's
-  // line once instead of once per 16 bytes
+  // line once instead of once per 16 bytes (volatile: without it the compiler
+  // may take a load whose address does not change out of a loop, past the
+  // alignment test)
   if constexpr (sizeof(T) * DP >= 32) {
     if (D == DP && (base & 31u) == 0) {
 #pragma unroll
       for (int v = 0; v < (int)(sizeof(T) * DP / 32); ++v) {
         const T *p = X + m * DP + v * (32 / (int)sizeof(T));
         if constexpr (sizeof(T) == 4) {
-          asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                        : "=f"(out[8 * v]), "=f"(out[8 * v + 1]), "=f"(out[8 * v + 2]), "=f"(out[8 * v + 3]),
                          "=f"(out[8 * v + 4]), "=f"(out[8 * v + 5]), "=f"(out[8 * v + 6]), "=f"(out[8 * v + 7])
                        : "l"(p));
         } else {
-          asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+          asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
                        : "=d"(out[4 * v]), "=d"(out[4 * v + 1]), "=d"(out[4 * v + 2]), "=d"(out[4 * v + 3])
                        : "l"(p));
         }
@@ -118,18 +120,22 @@ __device__ __forceinline__ void load_row(const T *__restrict__ X, int64_t m, int
 }
 
 // Cholesky of (scale P + S + jit I) in FP64 registers; false if a pivot is
-// not positive.  Padded dimensions are the identity.
-template <typename T, int DP>
-__device__ __forceinline__ bool chol_rows(const T (&S)[DP * (DP + 1) / 2], const T (&Pv)[DP * (DP + 1) / 2],
-                                          bool has_p, T scale, T jit, int D, double (&L)[DP * (DP + 1) / 2]) {
+// not positive.  Padded dimensions are the identity.  S (an entry by its
+// packed index) and the rows of P are taken one row at a time: with both held
+// beside L the posterior set the whole pass's registers.
+template <typename T, int DP, typename F>
+__device__ __forceinline__ bool chol_rows(F &&S, const T *__restrict__ P, T scale, T jit, int D,
+                                          double (&L)[DP * (DP + 1) / 2]) {
 #pragma unroll
-  for (int i = 0; i < DP; ++i)
+  for (int i = 0; i < DP; ++i) {
+    T row[DP];
+    if (P) load_row<T, DP>(P, i < D ? i : 0, D, row);
 #pragma unroll
     for (int j = 0; j <= i; ++j) {
       double v;
       if (i < D) {
-        T s = S[tix<DP>(i, j)];
-        if (has_p) s = f_add(f_mul(Pv[tix<DP>(i, j)], scale), s);
+        T s = S(tix<DP>(i, j));
+        if (P) s = f_add(f_mul(row[j], scale), s);
         if (i == j) s = f_add(s, jit);
         v = (double)s;
       } else {
@@ -137,6 +143,7 @@ __device__ __forceinline__ bool chol_rows(const T (&S)[DP * (DP + 1) / 2], const
       }
       L[tix<DP>(i, j)] = v;
     }
+  }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < DP; ++k) {
@@ -161,33 +168,20 @@ __device__ __forceinline__ bool chol_rows(const T (&S)[DP * (DP + 1) / 2], const
 // substitution, mm = nu trace and the b update; writes the per-kernel
 // outputs (NaN when the ladder failed or the row had an invalid index) and
 // returns whether L holds a factor.
-template <typename T, int DP>
-__device__ __forceinline__ bool row_posterior(const RowArgs<T> &g, int64_t n, const T (&S)[DP * (DP + 1) / 2], T nu,
-                                              bool bad, double (&L)[DP * (DP + 1) / 2], T &logdet) {
-  constexpr int TT = DP * (DP + 1) / 2;
+template <typename T, int DP, typename F>
+__device__ __forceinline__ bool row_posterior(const RowArgs<T> &g, int64_t n, F &&S, T nu, bool bad,
+                                              double (&L)[DP * (DP + 1) / 2], T &logdet) {
   const int D = g.D;
   const T b_old = g.b[n];
   const T scale = f_mul(g.nu0, f_div(g.a[n], b_old));
-  // the lower triangle of P_n, row by row (vector loads for D == DP)
-  T Pv[TT];
-  const bool has_p = g.P != nullptr;
-  if (has_p) {
-    const T *P = g.P + n * g.Pbs;
-#pragma unroll
-    for (int i = 0; i < DP; ++i) {
-      T row[DP];
-      load_row<T, DP>(P, i, D, row);
-#pragma unroll
-      for (int j = 0; j <= i; ++j) Pv[tix<DP>(i, j)] = i < D ? row[j] : T(0);
-    }
-  }
+  const T *P = g.P ? g.P + n * g.Pbs : nullptr;
   T jit = g.jitter[n];
-  bool ok = chol_rows<T, DP>(S, Pv, has_p, scale, jit, D, L);
+  bool ok = chol_rows<T, DP>(S, P, scale, jit, D, L);
   if (!ok) {
     T jt = T(0);
     for (int k = 0; k < 32 && !ok; ++k) {
       jt = f_add(jt, (T)(g.eps * ldexp(1.0, k)));
-      ok = chol_rows<T, DP>(S, Pv, has_p, scale, jt, D, L);
+      ok = chol_rows<T, DP>(S, P, scale, jt, D, L);
       if (ok) jit = jt;
     }
   }
@@ -296,7 +290,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && DP == 8) ? 3 : 1) vi_r
   const T nu = g.nu0 + vsum;
   double L[TT];
   T logdet;
-  const bool ok = row_posterior<T, DP>(g, n, S, nu, bad, L, logdet);
+  const bool ok = row_posterior<T, DP>(g, n, [&](int e) { return S[e]; }, nu, bad, L, logdet);
   const T nanv = T(NAN);
 
   // ---------------------------------------------------------------- E-step
@@ -371,8 +365,23 @@ struct RowSlot {
   static constexpr int VSUM = TT, BAD = TT + 1, RINV = TT - DP, CST = TT, EXPO = TT + 1, OK = TT + 2;
 };
 
-template <typename T, int DP, int LPR, int B>
-__global__ void __launch_bounds__(128, 3) vi_rows_lanes_kernel(RowArgs<T> g) {
+//
+// What bounds it is the latency of the gathers, so resident warps and pairs in
+// flight, which share the registers.  At DP = 8 in 32 bits 16 warps an SM with
+// B = 3 (128 registers) lead: 247 us at 200,000 rows of 8 dimensions and 50
+// neighbours, against 259 with B = 4, 299 at 12 warps with B = 4 (the former 168
+// registers) and 289 at 20 warps (spills).  Below DP = 8 the registers bind
+// nothing and B = 4 leads (circle rows of 2: 14.6 us, 16.2 with B = 3).
+template <typename T, int DP>
+struct RowPlan {
+  static constexpr bool WIDE = sizeof(T) == 4 && DP == 8;
+  static constexpr int BLOCKS = WIDE ? 4 : 3;                    // of 128 threads an SM
+  static constexpr int B = sizeof(T) == 8 ? 2 : WIDE ? 3 : 4;  // pairs in flight a lane
+};
+
+template <typename T, int DP, int LPR>
+__global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_kernel(RowArgs<T> g) {
+  constexpr int B = RowPlan<T, DP>::B;
   constexpr int TT = DP * (DP + 1) / 2;
   constexpr int GROUPS = 32 / LPR;
   constexpr unsigned FULL = 0xffffffffu;
@@ -466,14 +475,11 @@ __global__ void __launch_bounds__(128, 3) vi_rows_lanes_kernel(RowArgs<T> g) {
   {
     if (base + lane < g.N) {
       const int64_t n = own_n;
-      T S[TT];
-#pragma unroll
-      for (int e = 0; e < TT; ++e) S[e] = slot[lane][e];
       const T nu = g.nu0 + slot[lane][RS::VSUM];
       const bool bad = slot[lane][RS::BAD] != T(0);
       double L[TT];
       T logdet;
-      const bool ok = row_posterior<T, DP>(g, n, S, nu, bad, L, logdet);
+      const bool ok = row_posterior<T, DP>(g, n, [&](int e) { return slot[lane][e]; }, nu, bad, L, logdet);
 #pragma unroll
       for (int i = 0; i < DP; ++i) {
 #pragma unroll
@@ -622,18 +628,18 @@ extern "C" int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts, cons
     // 2 lanes per row for the pairs, a lane per row for the posterior (128
     // rows per 128-thread block; 8 lanes per row measured 10 % slower: more
     // passes of fewer rows each)
-    constexpr int LPR = 2, B = sizeof(TT) == 4 ? 4 : 2;
+    constexpr int LPR = 2;
     const int64_t blocks = (N + 127) / 128;
     if (blocks > 0x7fffffffLL) {
       set_error("vi_rows: too many rows");
       return (int)LAKDE_EUNSUPPORTED;
     }
     if (D <= 2)
-      vi_rows_lanes_kernel<TT, 2, LPR, B><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      vi_rows_lanes_kernel<TT, 2, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
     else if (D <= 4)
-      vi_rows_lanes_kernel<TT, 4, LPR, B><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      vi_rows_lanes_kernel<TT, 4, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
     else
-      vi_rows_lanes_kernel<TT, 8, LPR, B><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      vi_rows_lanes_kernel<TT, 8, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
     return check_launch("vi_rows");
   });
 }
