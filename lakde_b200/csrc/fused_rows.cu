@@ -61,26 +61,27 @@ __device__ __forceinline__ constexpr int tix(int i, int j) { return i * (i + 1) 
 // rows are DP * 4 or DP * 8 bytes apart and start 16-byte aligned (DP in
 // {4, 8}) or 8-byte aligned (DP = 2): vector loads, so a gather of one row per
 // thread is one or two load instructions instead of DP.
-template <typename T, int DP>
+// FIXED: the address is the same on every turn of a loop around the call.
+template <typename T, int DP, bool FIXED = false>
 __device__ __forceinline__ void load_row(const T *__restrict__ X, int64_t m, int D, T (&out)[DP]) {
   const uintptr_t base = reinterpret_cast<uintptr_t>(X);
   // rows of 32 bytes (or 64) from a 32-byte aligned base: one 256-bit load
   // per 32 bytes, so a warp's gather of scattered rows touches each row's
-  // line once instead of once per 16 bytes (volatile: without it the compiler
-  // may take a load whose address does not change out of a loop, past the
-  // alignment test)
-  if constexpr (sizeof(T) * DP >= 32) {
+  // line once instead of once per 16 bytes.  Not for an
+  // address that a loop does not change: the compiler may take the load, an
+  // asm statement, out of that loop and so past the alignment test
+  if constexpr (sizeof(T) * DP >= 32 && !FIXED) {
     if (D == DP && (base & 31u) == 0) {
 #pragma unroll
       for (int v = 0; v < (int)(sizeof(T) * DP / 32); ++v) {
         const T *p = X + m * DP + v * (32 / (int)sizeof(T));
         if constexpr (sizeof(T) == 4) {
-          asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                        : "=f"(out[8 * v]), "=f"(out[8 * v + 1]), "=f"(out[8 * v + 2]), "=f"(out[8 * v + 3]),
                          "=f"(out[8 * v + 4]), "=f"(out[8 * v + 5]), "=f"(out[8 * v + 6]), "=f"(out[8 * v + 7])
                        : "l"(p));
         } else {
-          asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+          asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
                        : "=d"(out[4 * v]), "=d"(out[4 * v + 1]), "=d"(out[4 * v + 2]), "=d"(out[4 * v + 3])
                        : "l"(p));
         }
@@ -129,7 +130,7 @@ __device__ __forceinline__ bool chol_rows(F &&S, const T *__restrict__ P, T scal
 #pragma unroll
   for (int i = 0; i < DP; ++i) {
     T row[DP];
-    if (P) load_row<T, DP>(P, i < D ? i : 0, D, row);
+    if (P) load_row<T, DP, true>(P, i < D ? i : 0, D, row);
 #pragma unroll
     for (int j = 0; j <= i; ++j) {
       double v;
@@ -368,7 +369,7 @@ struct RowSlot {
 //
 // What bounds it is the latency of the gathers, so resident warps and pairs in
 // flight, which share the registers.  At DP = 8 in 32 bits 16 warps an SM with
-// B = 3 (128 registers) lead: 247 us at 200,000 rows of 8 dimensions and 50
+// B = 3 (128 registers) lead: 250 us at 200,000 rows of 8 dimensions and 50
 // neighbours, against 259 with B = 4, 299 at 12 warps with B = 4 (the former 168
 // registers) and 289 at 20 warps (spills).  Below DP = 8 the registers bind
 // nothing and B = 4 leads (circle rows of 2: 14.6 us, 16.2 with B = 3).
