@@ -45,6 +45,16 @@ def calc_log_rho_block(X_test, X_train, nu, W_triu, logdet_W):
     return Q
 
 
+# The block schedule's dense E-step takes a kernel block against this many
+# (kernel, point) entries at once, in whole blocks of points: 128 MB of log rho
+# in float32.  A step over one block of points at a time is 25 launches and a
+# synchronisation each, however small the block: an iteration on 2,000 points
+# of 2 dimensions in blocks of 512 took 10.5 ms so and 5.5 ms with one step a
+# kernel block.  Tens of millions of entries fill the GPU; more would only hold
+# more memory.
+DENSE_ENTRIES = 1 << 25
+
+
 class LocallyAdaptiveKDE(VIModel, ABC):
     def __init__(self, nu_0, a_0, b_0, block_size, verbose, logs, fused=False, candidates="knn", cuda_graph=True):
         super().__init__(block_size, verbose, logs)
@@ -72,6 +82,19 @@ class LocallyAdaptiveKDE(VIModel, ABC):
         s = block_idx * self.block_size
         return s, s + self.block_size
 
+    def _log_rho_slabs(self, X, block_idx, nu, W_triu, logdet_W):
+        """(points slice, log rho of the kernel block against them), own pairs -inf."""
+        N = X.size(0)
+        s, e = self._span(block_idx)
+        rows = X[s:e]
+        step = self.block_size * max(1, DENSE_ENTRIES // (self.block_size * rows.size(0)))
+        for j in range(0, N, step):
+            sl = slice(j, min(j + step, N))
+            log_rho = calc_log_rho_block(X[sl], rows, nu, W_triu, logdet_W)
+            if j <= s < sl.stop:
+                log_rho[:, s - j : e - j].diagonal().fill_(-math.inf)
+            yield sl, log_rho
+
     def calc_posterior_contribs(self, X, block_idx):
         """S and nu of one kernel block from its COO (lakde/local_adaptive_kde.py:66-81)."""
         s, e = self._span(block_idx)
@@ -96,37 +119,34 @@ class LocallyAdaptiveKDE(VIModel, ABC):
     def partial_expectation_step(self, X, block_idx, W_triu, nu, update_normalization=True, sparsity_threshold=None):
         """Dense E-step of one kernel block against all points (lakde/local_adaptive_kde.py:98-154)."""
         N, D = X.shape
-        s, e = self._span(block_idx)
-        X_train = X[s:e]
         logdet_W = chol_logdet(W_triu)
         rnm_log_consts = self.rnm_log_consts
         old_log_consts = rnm_log_consts
-        blocks = []
+        blocks, widths = [], []
         if update_normalization:
             rnm_log_consts = rnm_log_consts.clone()
             (_, col), values = self.rnm_blocks[block_idx]
             old_sums = X.new_zeros(N).scatter_add_(0, col.long(), values)
             old_contribs = torch.log(old_sums) + old_log_consts
-        for bj, j in enumerate(range(0, N, self.block_size)):
-            X_test = X[j : j + self.block_size]
-            log_rho = calc_log_rho_block(X_test, X_train, nu, W_triu, logdet_W)
-            if block_idx == bj:
-                log_rho.diagonal().fill_(-math.inf)
+        for sl, log_rho in self._log_rho_slabs(X, block_idx, W_triu=W_triu, nu=nu, logdet_W=logdet_W):
             if update_normalization:
-                sl = slice(j, j + self.block_size)
                 torch.logaddexp(
                     logsubexp(old_log_consts[sl], old_contribs[sl]),
                     torch.logsumexp(log_rho, dim=0),
                     out=rnm_log_consts[sl],
                 )
-            r = torch.exp_(log_rho.sub_(rnm_log_consts[j : j + self.block_size]))
+            r = torch.exp_(log_rho.sub_(rnm_log_consts[sl]))
             if sparsity_threshold:
                 r = torch.threshold_(r, sparsity_threshold, 0)
             idx = torch.nonzero(r).T.contiguous()
             blocks.append((idx.to(torch.int32), r[idx.unbind()]))
-        indices, values = cat_sparse(*zip(*blocks), self.block_size, dim=1)
-        perm = torch.argsort(indices[0].long() * N + indices[1].long())
-        indices, values = indices[:, perm], values[perm]
+            widths.append(r.size(1))
+        if len(blocks) == 1:  # nonzero lists its entries in (row, column) order
+            indices, values = blocks[0]
+        else:
+            indices, values = cat_sparse(*zip(*blocks), widths, dim=1)
+            perm = torch.argsort(indices[0].long() * N + indices[1].long())
+            indices, values = indices[:, perm], values[perm]
         if update_normalization:
             return indices, values, rnm_log_consts
         return indices, values
@@ -137,18 +157,16 @@ class LocallyAdaptiveKDE(VIModel, ABC):
         finfo = torch.finfo(X.dtype)
         coeff = torch.clamp_(torch.exp(self.rnm_log_consts - rnm_log_consts), min=finfo.tiny, max=finfo.max)
         sums = X.new_zeros(N)
-        for bi in range(len(self.rnm_blocks)):
-            (_, col), values = self.rnm_blocks[bi]
-            col = col.long()
+        cols = [ind[1].long() for ind, _ in self.rnm_blocks]
+        for bi, (col, (_, values)) in enumerate(zip(cols, self.rnm_blocks)):
             if bi != block_idx:
                 values *= coeff[col]
             sums.scatter_add_(0, col, values)
         sums = torch.clamp_min(sums, finfo.eps)
         rnm_log_consts += sums.log()
         coeff = torch.clamp_(torch.reciprocal(sums), min=finfo.tiny, max=finfo.max)
-        for bi in range(len(self.rnm_blocks)):
-            (_, col), values = self.rnm_blocks[bi]
-            values *= coeff[col.long()]
+        for col, (_, values) in zip(cols, self.rnm_blocks):
+            values *= coeff[col]
         return rnm_log_consts
 
     # ------------------------------------------------------------- fused path

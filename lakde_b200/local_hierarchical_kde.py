@@ -12,7 +12,6 @@ from .engine import FusedHier, build_pattern
 from .linalg_util import chol_logdet, chol_mm_trace, mvdigamma, mvlgamma, stabilized_cholesky, tril_inverse
 from .local_adaptive_kde import (
     LocallyAdaptiveKDE,
-    calc_log_rho_block,
     expect_log_p_tau,
     expect_log_q_tau,
 )
@@ -158,7 +157,6 @@ class LocalHierarchicalKDE(LocallyAdaptiveKDE):
         N = X.size(0)
         sigma_bar, _ = self.calc_prior_cov()
         for bi, i in enumerate(range(0, N, self.block_size)):
-            X_train = X[i : i + self.block_size]
             S, nu = self.calc_posterior_contribs(X, bi)
             W_triu = self.calc_posterior(bi, sigma_bar, S)
             logdet_W = chol_logdet(W_triu)
@@ -166,11 +164,7 @@ class LocalHierarchicalKDE(LocallyAdaptiveKDE):
             self.nu[sl] = nu
             self.logdet_W[sl] = logdet_W
             self.expect_lambda_contribs[bi] = self._expect_lambda_contrib(W_triu, nu, self.a[sl] / self.b[sl])
-            for bj, j in enumerate(range(0, N, self.block_size)):
-                log_rho = calc_log_rho_block(X[j : j + self.block_size], X_train, nu, W_triu, logdet_W)
-                if bi == bj:
-                    log_rho.diagonal().fill_(-math.inf)
-                jl = slice(j, j + self.block_size)
+            for jl, log_rho in self._log_rho_slabs(X, bi, nu, W_triu, logdet_W):
                 torch.logaddexp(self.rnm_log_consts[jl], torch.logsumexp(log_rho, dim=0), out=self.rnm_log_consts[jl])
         for bi in range(self.num_blocks(N)):
             S, nu = self.calc_posterior_contribs(X, bi)

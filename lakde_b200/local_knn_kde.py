@@ -11,7 +11,6 @@ from .engine import FusedKNN, build_pattern
 from .linalg_util import chol_logdet, chol_mm_trace, mvdigamma, mvlgamma, stabilized_cholesky
 from .local_adaptive_kde import (
     LocallyAdaptiveKDE,
-    calc_log_rho_block,
     expect_log_p_tau,
     expect_log_q_tau,
 )
@@ -146,7 +145,6 @@ class LocalKNearestKDE(LocallyAdaptiveKDE):
             return
         N = X.size(0)
         for bi, i in enumerate(range(0, N, self.block_size)):
-            X_train = X[i : i + self.block_size]
             sigma_0, sigma_0_tril = self.calc_prior_cov(X, bi)
             S, nu = self.calc_posterior_contribs(X, bi)
             W_triu = self.calc_posterior(bi, sigma_0, S)
@@ -156,11 +154,7 @@ class LocalKNearestKDE(LocallyAdaptiveKDE):
             self.logdet_W[sl] = logdet_W
             self.logdet_sigma_0[sl] = chol_logdet(sigma_0_tril)
             self.sigma_0_lambda_mm_trace[sl] = nu * chol_mm_trace(sigma_0_tril, W_triu)
-            for bj, j in enumerate(range(0, N, self.block_size)):
-                log_rho = calc_log_rho_block(X[j : j + self.block_size], X_train, nu, W_triu, logdet_W)
-                if bi == bj:
-                    log_rho.diagonal().fill_(-math.inf)
-                jl = slice(j, j + self.block_size)
+            for jl, log_rho in self._log_rho_slabs(X, bi, nu, W_triu, logdet_W):
                 torch.logaddexp(self.rnm_log_consts[jl], torch.logsumexp(log_rho, dim=0), out=self.rnm_log_consts[jl])
         for bi in range(self.num_blocks(N)):
             sigma_0, _ = self.calc_prior_cov(X, bi)
