@@ -3,6 +3,7 @@
 //   chol_quad_form  — dense Cholesky quad forms (the sweep of sweep.cuh)
 //   W_inv           — CSR responsibility-weighted scatter covariance (M-step)
 #include "common.cuh"
+#include "factor_dmma.cuh"
 #include "sweep.cuh"
 
 namespace lakde {
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(256) scatter_cov_warp(const RP *__restrict__ r
 }
 
 // ---------------------------------------------------------------------------
-// Scatter covariance, D in (16, 64]: one CTA per kernel row; each thread owns
+// Scatter covariance in float32, D in (16, 64]: one CTA per kernel row; each thread owns
 // one 4x4 block of the lower triangle and updates it from 64-pair chunks of
 // centred differences staged in shared memory (two 16-byte loads per pair).
 // ---------------------------------------------------------------------------
@@ -271,6 +272,121 @@ __global__ void scatter_cov_cta(const RP *__restrict__ rowptr, const CI *__restr
       o[i * D + j] = v;
       o[j * D + i] = v;
     }
+}
+
+// ---------------------------------------------------------------------------
+// Scatter covariance in float64, D in (16, 64]: one warp per kernel row on the
+// FP64 tensor cores, the lower 8 x 8 tiles of S_n in registers.  A step takes
+// four pairs: lane l gathers the entries 8 I + l / 4 of pair l % 4's point,
+// whose centred differences are the A fragment of row block I and, times the
+// weight, the B fragment of column block I, so nothing passes through shared
+// memory; the next step's gather is in flight under a step's products.
+// Blocks of one warp: with several rows a block, the short ones wait for the
+// longest.
+//
+// Bound by the FP64 tensor pipe (NT (NT + 1) / 2 MMAs of 16 cycles a step) and
+// the gather from L2.  20,000 rows of 80 pairs on average at d = 43: 698 -> 259
+// us, the tensor pipe 46 % busy (a fifth of the time is the longest rows' tail);
+// d = 63 1278 -> 450, d = 24 2211 -> 121 (the CTA form above, whose 4 x 4
+// register blocks read both operands from shared memory; it stays for float32,
+// where the FP32 pipe has twice the rate: 417 us at d = 43).
+// ---------------------------------------------------------------------------
+template <typename RP, typename CI, int DP>
+__global__ void __launch_bounds__(32, DP <= 32 ? 16 : DP <= 48 ? 12 : 8)
+    scatter_cov_mma(const RP *__restrict__ rowptr, const CI *__restrict__ col, const double *__restrict__ val,
+                    const double *__restrict__ Xn, const double *__restrict__ Xm, double *__restrict__ out, int64_t M,
+                    int D, double *__restrict__ nu_out, double nu0) {
+  constexpr int NT = DP / 8;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+  const int64_t row = blockIdx.x;
+  const int64_t start = (int64_t)rowptr[row], end = (int64_t)rowptr[row + 1];
+  bool bad = end < start;
+
+  double xn[NT];
+#pragma unroll
+  for (int I = 0; I < NT; ++I) xn[I] = 8 * I + g < D ? Xn[row * D + 8 * I + g] : 0.0;
+  double c[NT * (NT + 1) / 2][2];
+#pragma unroll
+  for (int e = 0; e < NT * (NT + 1) / 2; ++e) c[e][0] = c[e][1] = 0.0;
+  double vsum = 0.0;
+
+  // pair base + lane of 32: its point (-1: none) and weight; the next 32's are loaded ahead
+  int64_t ci = -1, ci1 = -1;
+  double v = 0.0, v1 = 0.0;
+  auto load_pairs = [&](int64_t base) {
+    const int64_t p = base + lane;
+    ci1 = -1;
+    v1 = 0.0;
+    if (p < end) {
+      ci1 = (int64_t)col[p];
+      v1 = val[p];
+    }
+  };
+  auto take_pairs = [&](int64_t base) {
+    ci = ci1;
+    v = v1;
+    if (base + lane < end && (ci < 0 || ci >= M)) {
+      bad = true;
+      ci = -1;
+      v = 0.0;
+    }
+    vsum += v;
+    load_pairs(base + 32);
+  };
+  double x[NT], w;
+  bool ok;
+  auto gather = [&](int s) {  // pairs 4 s .. 4 s + 3 of the 32
+    const int64_t cs = __shfl_sync(FULL, ci, 4 * s + t);
+    w = __shfl_sync(FULL, v, 4 * s + t);
+    ok = cs >= 0;
+#pragma unroll
+    for (int I = 0; I < NT; ++I) x[I] = ok && 8 * I + g < D ? Xm[cs * D + 8 * I + g] : 0.0;
+  };
+  if (start < end) {
+    load_pairs(start);
+    take_pairs(start);
+    gather(0);
+    for (int64_t p = start; p < end;) {
+      double dl[NT], b[NT];
+#pragma unroll
+      for (int I = 0; I < NT; ++I) {
+        dl[I] = ok ? x[I] - xn[I] : 0.0;
+        b[I] = w * dl[I];
+      }
+      p += 4;
+      if (p < end) {
+        const int s = (int)((p - start) >> 2) & 7;
+        if (s == 0) take_pairs(p);
+        gather(s);
+      }
+#pragma unroll
+      for (int I = 0; I < NT; ++I)
+#pragma unroll
+        for (int J = 0; J <= I; ++J) {
+          double *t = c[I * (I + 1) / 2 + J];
+          dmma::mma(t[0], t[1], dl[I], b[J]);
+        }
+    }
+  }
+  bad = __any_sync(FULL, bad);
+  if (nu_out) {
+    vsum = warp_sum(vsum);
+    if (lane == 0) nu_out[row] = bad ? (double)NAN : nu0 + vsum;
+  }
+  double *o = out + row * (int64_t)D * D;
+#pragma unroll
+  for (int I = 0; I < NT; ++I)
+#pragma unroll
+    for (int J = 0; J <= I; ++J)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = 8 * I + g, j = 8 * J + 2 * t + h;
+        if (i >= D || j > i) continue;
+        const double s = bad ? (double)NAN : c[I * (I + 1) / 2 + J][h];
+        o[i * D + j] = s;
+        o[j * D + i] = s;
+      }
 }
 
 template <typename K>
@@ -388,6 +504,9 @@ static int scatter_cov_launch(const char *what, int dtype, const void *rowptr, i
             const int64_t blocks = (N + 7) / 8;
             scatter_cov_warp<T, RP, CI, DP><<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
                 rp, cp, vp, xn, xm, op, N, M, (int)D, static_cast<T *>(nu_out), (T)nu0);
+          } else if constexpr (sizeof(T) == 8) {
+            scatter_cov_mma<RP, CI, DP><<<(unsigned)N, 32, 0, as_stream(stream)>>>(rp, cp, vp, xn, xm, op, M, (int)D,
+                                                                                   static_cast<T *>(nu_out), (T)nu0);
           } else {
             using C = CtaScatterCfg<T, DP>;
             auto kern = scatter_cov_cta<T, RP, CI, DP>;
