@@ -347,16 +347,16 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && DP == 8) ? 3 : 1) vi_r
 }
 
 // The same pass with the pairs of a kernel row dealt to a group of LPR lanes
-// and the FP64 posterior one row per lane.  A warp takes 32 consecutive rows
+// and the FP64 posterior one row per lane.  A warp takes RW consecutive rows
 // of the order, 32 / LPR rows at a time in the M- and E-steps: a row's pairs
 // go to the group's lanes (pair start + l + LPR k to lane l, so the index,
 // responsibility and log rho accesses of a warp are coalesced), in batches of
 // B whose gathers are all in flight together.  An xor butterfly sums the
 // group's shares of S_n and sum r (every lane ends with the same bits, in a
 // fixed order) and lane 0 of the group parks them in the row's slot of the
-// warp's shared memory.  Posterior: lane l factorises row l from its slot
-// (all 32 lanes on the FP64 work) and parks the factor's pieces in the same
-// slot, which the groups read back for the E-step.
+// warp's shared memory.  Posterior: lane l < RW factorises row l from its slot
+// and parks the factor's pieces in the same slot, which the groups read back
+// for the E-step.
 template <typename T, int DP>
 struct RowSlot {
   static constexpr int TT = DP * (DP + 1) / 2;
@@ -372,7 +372,8 @@ struct RowSlot {
 // B = 3 (128 registers) lead: 250 us at 200,000 rows of 8 dimensions and 50
 // neighbours, against 259 with B = 4, 299 at 12 warps with B = 4 (the former 168
 // registers) and 289 at 20 warps (spills).  Below DP = 8 the registers bind
-// nothing and B = 4 leads (circle rows of 2: 14.6 us, 16.2 with B = 3).
+// nothing and B = 4 leads (2,000 rows of 2: 14.6 us at 32 rows a warp, 16.2
+// with B = 3).
 template <typename T, int DP>
 struct RowPlan {
   static constexpr bool WIDE = sizeof(T) == 4 && DP == 8;
@@ -380,22 +381,23 @@ struct RowPlan {
   static constexpr int B = sizeof(T) == 8 ? 2 : WIDE ? 3 : 4;  // pairs in flight a lane
 };
 
-template <typename T, int DP, int LPR>
+template <typename T, int DP, int LPR, int RW>
 __global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_kernel(RowArgs<T> g) {
   constexpr int B = RowPlan<T, DP>::B;
   constexpr int TT = DP * (DP + 1) / 2;
-  constexpr int GROUPS = 32 / LPR;
+  constexpr int GROUPS = 32 / LPR, PASSES = RW / GROUPS;
   constexpr unsigned FULL = 0xffffffffu;
   using RS = RowSlot<T, DP>;
-  __shared__ T park[4][32][RS::SIZE];
+  __shared__ T park[4][RW][RS::SIZE];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (LPR - 1), grp = lane / LPR;
-  const int64_t base = ((int64_t)blockIdx.x * 4 + warp) * 32;
+  const int64_t base = ((int64_t)blockIdx.x * 4 + warp) * RW;
   T(*slot)[RS::SIZE] = park[warp];
   const int D = g.D;
   // each lane loads the setup of one of the warp's rows (row index, pair
   // range, its point row); the groups take their row's from that lane
   int64_t own_n = 0, own_start = 0, own_end = 0;
-  if (base + lane < g.N) {
+  const bool own = lane < RW && base + lane < g.N;
+  if (own) {
     own_n = g.order ? (int64_t)g.order[base + lane] : base + lane;
     own_start = g.rowptr[own_n];
     own_end = g.rowptr[own_n + 1];
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_ker
 
   // ---------------------------------------------------------------- M-step
 #pragma unroll 1
-  for (int pass = 0; pass < LPR; ++pass) {
+  for (int pass = 0; pass < PASSES; ++pass) {
     const int rl = pass * GROUPS + grp;
     const int64_t n = __shfl_sync(FULL, own_n, rl);
     const int64_t start = __shfl_sync(FULL, own_start, rl);
@@ -474,7 +476,7 @@ __global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_ker
 
   // ------------------------------------------------------ posterior, a lane per row
   {
-    if (base + lane < g.N) {
+    if (own) {
       const int64_t n = own_n;
       const T nu = g.nu0 + slot[lane][RS::VSUM];
       const bool bad = slot[lane][RS::BAD] != T(0);
@@ -498,7 +500,7 @@ __global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_ker
   // ---------------------------------------------------------------- E-step
   const T nanv = T(NAN);
 #pragma unroll 1
-  for (int pass = 0; pass < LPR; ++pass) {
+  for (int pass = 0; pass < PASSES; ++pass) {
     const int rl = pass * GROUPS + grp;
     const int64_t n = __shfl_sync(FULL, own_n, rl);
     const int64_t start = __shfl_sync(FULL, own_start, rl);
@@ -626,21 +628,37 @@ extern "C" int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts, cons
         vi_rows_kernel<TT, 8><<<blocks, 128, 0, as_stream(stream)>>>(g);
       return check_launch("vi_rows");
     }
-    // 2 lanes per row for the pairs, a lane per row for the posterior (128
-    // rows per 128-thread block; 8 lanes per row measured 10 % slower: more
-    // passes of fewer rows each)
-    constexpr int LPR = 2;
-    const int64_t blocks = (N + 127) / 128;
-    if (blocks > 0x7fffffffLL) {
-      set_error("vi_rows: too many rows");
-      return (int)LAKDE_EUNSUPPORTED;
-    }
-    if (D <= 2)
-      vi_rows_lanes_kernel<TT, 2, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
-    else if (D <= 4)
-      vi_rows_lanes_kernel<TT, 4, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
-    else
-      vi_rows_lanes_kernel<TT, 8, LPR><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
-    return check_launch("vi_rows");
+    // Rows a warp and lanes a row, by the number of rows.  One warp's chain
+    // (index and point loads of each pass, the FP64 posterior) takes the same
+    // time with 2 rows as with 32, so rows are packed only as far as the chip is
+    // full without: 2, 4, 8, 16 and 32 rows a warp cross at 1,500 to 4,500
+    // warps (the wider passes take longer).  Measured at 2 / 4 / 8 / 16 / 32
+    // rows, us: float32 d = 2, K = 20: 2,000 rows 6.6 / 6.8 / 7.6 / 10.2 / 15.0,
+    // 20,000 rows 21.8 / 14.9 / 10.7 / 13.2 / 18.5; d = 8, K = 50: 2,000 rows
+    // 24 / 26 / 33 / 51 / 83, 10,000 rows 71 / 52 / 42 / 60 / 95, 40,000 rows
+    // 231 / 136 / 90 / 73 / 111, 200,000 rows 1208 / 667 / 391 / 298 / 249;
+    // float64 d = 8: 3,000 rows 29 / 34 / 46 / 73 / 126, 60,000 rows 458 / 275
+    // / 185 / 145 / 183.
+    auto launch = [&](auto lpr, auto rw) {
+      constexpr int LPR = decltype(lpr)::value, RW = decltype(rw)::value;
+      const int64_t blocks = (N + 4 * RW - 1) / (4 * RW);
+      if (blocks > 0x7fffffffLL) {
+        set_error("vi_rows: too many rows");
+        return (int)LAKDE_EUNSUPPORTED;
+      }
+      if (D <= 2)
+        vi_rows_lanes_kernel<TT, 2, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      else if (D <= 4)
+        vi_rows_lanes_kernel<TT, 4, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      else
+        vi_rows_lanes_kernel<TT, 8, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+      return check_launch("vi_rows");
+    };
+    using std::integral_constant;
+    if (N <= 3000) return launch(integral_constant<int, 16>{}, integral_constant<int, 2>{});
+    if (N <= 8000) return launch(integral_constant<int, 8>{}, integral_constant<int, 4>{});
+    if (N <= 24000) return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{});
+    if (N <= 72000) return launch(integral_constant<int, 2>{}, integral_constant<int, 16>{});
+    return launch(integral_constant<int, 2>{}, integral_constant<int, 32>{});
   });
 }
