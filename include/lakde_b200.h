@@ -394,6 +394,13 @@ LAKDE_API int lakde_mstep_tc_tiled(int dtype, int64_t N, int64_t D, int64_t npts
                                    void *stream);
 
 /*
+ * failed[0] = min(failed[0], info_0, ..., info_{N-1}): the worst factorisation
+ * status of a fit, kept on the device (0 while every matrix factorised).
+ */
+LAKDE_API int lakde_fold_info(int64_t N, const int32_t *info, int32_t *failed,
+                              void *stream);
+
+/*
  * lakde_posterior_factor from tiled inputs: A_n = nu_0 a_n / b_n P_n + S_n
  * with S_n and P_n from SP, and the trace term from the lower triangular T_n
  * as tiles (T_tiles, 64 * tiles floats per kernel, may be NULL).  float32,

@@ -105,6 +105,7 @@ _SIGNATURES = {
         [_c_vp, _c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_int, _c_i64, _c_int, _c_vp, _c_int, _c_vp, _c_vp],
         _c_int,
     ),
+    "lakde_fold_info": ([_c_i64, _c_vp, _c_vp, _c_vp], _c_int),
     "lakde_tile_count": ([_c_i64], _c_i64),
     "lakde_pack_tiles": ([_c_int, _c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_i64, _c_i64, _c_i64, _c_vp], _c_int),
     "lakde_mstep_tc_tiled": (

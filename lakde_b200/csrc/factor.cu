@@ -723,6 +723,17 @@ __global__ void __launch_bounds__(32 * DmmaCfg<DP, LEAN>::WPB, DmmaCfg<DP, LEAN>
   }
 }
 
+// failed = min(failed, min_n info_n): one pass with an atomic only where a
+// status is negative (a reduction and a minimum as two launches took 4 of an
+// iteration's 26 us at 2,000 rows).
+__global__ void __launch_bounds__(256) fold_info_kernel(const int32_t *__restrict__ info, int64_t N,
+                                                        int32_t *__restrict__ failed) {
+  int32_t worst = 0;
+  for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x)
+    worst = min(worst, info[n]);
+  if (worst < 0) atomicMin(failed, worst);
+}
+
 }  // namespace lakde
 
 using namespace lakde;
@@ -829,6 +840,24 @@ extern "C" int lakde_posterior_factor(int dtype, int64_t N, int64_t D, const voi
 }
 
 // ------------------------------------------------------------- tiled layout
+extern "C" int lakde_fold_info(int64_t N, const int32_t *info, int32_t *failed, void *stream) {
+  clear_error();
+  if (N < 0) {
+    set_error("fold_info: invalid size (N=%lld)", (long long)N);
+    return LAKDE_EINVAL;
+  }
+  if (N == 0) return LAKDE_OK;
+  if (!info || !failed) {
+    set_error("fold_info: null pointer");
+    return LAKDE_EINVAL;
+  }
+  if (int st = bind_device("fold_info", {failed, info})) return st;
+  // a few statuses a thread, at most two blocks an SM
+  const int64_t blocks = (N + 1023) / 1024;
+  fold_info_kernel<<<(unsigned)(blocks < 296 ? blocks : 296), 256, 0, as_stream(stream)>>>(info, N, failed);
+  return check_launch("fold_info");
+}
+
 extern "C" int64_t lakde_tile_count(int64_t D) {
   int64_t nt = 0;
   if (D >= 1 && D <= kMaxDim) {

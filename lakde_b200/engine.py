@@ -181,7 +181,7 @@ class FusedVI:
             K.posterior_factor_tiled(self.SP, self.D, self.W_inv_jitter, self.eps, self.nu_0_t, self.a, self.b,
                                      None, self.logdet_W, self.info, T_tiles=Tt,
                                      trace=self.trace if with_trace else None, W_cores=self.Wc)
-            torch.minimum(self.failed, self.info.min(), out=self.failed)
+            K.fold_info(self.info, self.failed)
             return
         P, T = self._prior()
         K.posterior_factor(
@@ -189,7 +189,7 @@ class FusedVI:
             T=T if with_trace else None, info=self.info, out=self.U, logdet=self.logdet_W,
             trace=self.trace if with_trace else None, T_lower=self._T_lower, W_cores=self.Wc if mixed else None,
         )
-        torch.minimum(self.failed, self.info.min(), out=self.failed)
+        K.fold_info(self.info, self.failed)
 
     def estep_numerators(self):
         """log rho of every pair of the pattern (the E-step before the normaliser)."""
@@ -246,7 +246,7 @@ class FusedVI:
                 P, _ = self._prior()
                 K.posterior_factor(self.S, self.W_inv_jitter, self.eps, P=P, nu_0=self.nu_0_t, a=self.a, b=self.b,
                                    info=info, out=self.U, logdet=logdet, W_cores=self.Wc)
-            torch.minimum(self.failed, info.min(), out=self.failed)
+            K.fold_info(info, self.failed)
             lc = K.pred_coeff(nu, logdet, self.D)
             return K.log_pred_density_tc(self.Xp, self.Wc, nu, lc, Y.to(self.dtype), self.err)
         # S and W_triu into the engine's own buffers (the next step rewrites them first)
@@ -254,7 +254,7 @@ class FusedVI:
         P, _ = self._prior()
         K.posterior_factor(self.S, self.W_inv_jitter, self.eps, P=P, nu_0=self.nu_0_t, a=self.a, b=self.b,
                            logdet=logdet, info=info, out=self.U)
-        torch.minimum(self.failed, info.min(), out=self.failed)
+        K.fold_info(info, self.failed)
         lc = K.pred_coeff(nu, logdet, self.D)
         return K.log_pred_density(self.X, self.U, nu, lc, Y.to(self.dtype))
 
@@ -307,7 +307,7 @@ class FusedKNN(FusedVI):
 
         sigma_0 = batched_knn_cov(self.X, self.X, self.knn_graph.long())
         _, logdet_inv, info, L0, _ = K.posterior_factor(sigma_0, self.sigma_0_jitter, self.eps, want_L=True)
-        torch.minimum(self.failed, info.min(), out=self.failed)
+        K.fold_info(info, self.failed)
         self.logdet_sigma_0.copy_(-logdet_inv)
         sigma_0.diagonal(dim1=-2, dim2=-1).add_(self.sigma_0_jitter[:, None])
         self.sigma_0 = sigma_0
@@ -365,7 +365,7 @@ class FusedKNN(FusedVI):
             K.vi_rows(p.rowptr, p.col, self.r, self.X, self.nu_0, self.a, self.b, self.b_0_f, self.W_inv_jitter,
                       self.eps, self.nu, self.logdet_W, self.info, self.logrho, P=self.sigma_0, T=self.sigma_0_tril,
                       order=p.order, mm=self.sigma_0_lambda_mm_trace)
-            torch.minimum(self.failed, self.info.min(), out=self.failed)
+            K.fold_info(self.info, self.failed)
             K.estep_normalise(p.cptr, p.pos, self.logrho, self.r, self.c, self.rsum, 1, self.threshold)
             return
         self.refresh_points()
@@ -464,7 +464,7 @@ class FusedHier(FusedVI):
         prec = (self.expect_lambda_contribs.sum(0) * self.nu_0 + self.nu_shared_0 * self.lambda_0).unsqueeze(0)
         W_sh, _, info, _, _ = K.posterior_factor(prec.contiguous(), self.W_shared_inv_jitter,
                                                  torch.finfo(torch.float64).eps)
-        torch.minimum(self.failed, info.min(), out=self.failed)
+        K.fold_info(info, self.failed)
         self.W_shared_triu.copy_(W_sh[0])
         # E[Sigma_bar] follows the shared factor at once, so the next step and
         # log_pred_density both see the current prior

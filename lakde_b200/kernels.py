@@ -426,6 +426,14 @@ def posterior_factor_tiled(SP, D, jitter, eps, nu_0, a, b, out, logdet, info, T_
     )
 
 
+def fold_info(info, failed):
+    """failed = min(failed, min(info)) on the device (both int32; see include/lakde_b200.h)."""
+    nat.require_cuda(info, failed, op="fold_info")
+    assert info.dtype == torch.int32 and failed.dtype == torch.int32 and info.is_contiguous()
+    nat.check(nat.lib().lakde_fold_info(info.numel(), nat.ptr(info), nat.ptr(failed), nat.stream_of(failed)),
+              "fold_info")
+
+
 def weighted_gram(W_triu, w, out=None, workspace=None):
     """sum_n w_n W_triu_n W_triu_n^T in float64, [D, D] (see include/lakde_b200.h)."""
     nat.require_cuda(W_triu, w, out, op="weighted_gram")
