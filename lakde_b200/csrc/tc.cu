@@ -305,7 +305,7 @@ struct Cfg {
 // mbarriers (8 bytes each from Cfg::BAR)
 struct Bars {
   static constexpr int PFULL = 0;          // [2] a half of the plan written (the planner)
-  static constexpr int PEMPTY = 2;         // [2] ... and its last tile done with (converter, epilogue and copy warps)
+  static constexpr int PEMPTY = 2;         // [2] ... and its last tile done with (converter, epilogue, MMA and copy warps)
   static constexpr int MFULL = 4;          // [NS] indices of a slot written (32 lanes of its index warp)
   static constexpr int MEMPTY = MFULL + NS;  // [NS] slot free again (converter and epilogue warps)
   static constexpr int BFULL = MEMPTY + NS;  // [2] W cores of a B stage landed (every copy-warp lane)
@@ -903,7 +903,7 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(pfull + i, 1);
-      mbar_init(pempty + i, NCW + NEW + (MODE == MSTEP ? 0 : NCOPY));
+      mbar_init(pempty + i, NCW + NEW + 1 + (MODE == MSTEP ? 0 : NCOPY));
       mbar_init(bfull + i, 32 * NCOPY);
       mbar_init(bempty + i, 1);
       mbar_init(mma_done + i, 1);
@@ -937,7 +937,9 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
   if (warp == WARP_MMA) {
     // ----------------------------------------------------------- MMA warp
     // No wait on the plan but the first: the converters have seen the plan of
-    // tile t + 1 before they arrive for tile t.
+    // tile t + 1 before they arrive for tile t.  It does say when it has read an
+    // entry: the M-step's other warps can be done with a tile that does not end
+    // its row while this warp still waits for the tile before.
     int last = -1;  // last tile whose MMAs were issued
     bool ok = planned(0);
     for (int t = 0; ok; ++t) {
@@ -946,6 +948,7 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
       const int cnt = __shfl_sync(0xffffffffu, meta.cnt, 0), flags = __shfl_sync(0xffffffffu, meta.flags, 0);
       const int row = __shfl_sync(0xffffffffu, meta.row, 0);
       if (__shfl_sync(0xffffffffu, (int)(meta.n < 0), 0)) break;
+      if (lane == 0) unplan(t);
       if (flags & 1) {
         if (MODE != MSTEP) ok = mbar_wait(bfull + (row & 1), (uint32_t)((row >> 1) & 1));
         // the accumulator of row - 2 read

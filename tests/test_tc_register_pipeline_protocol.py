@@ -39,13 +39,17 @@ class Bar:
         return (self.completed & 1) != parity
 
 
-def simulate(rows, mode, na, seed, ncw=8, new=8, stall=False, early_release=False):
-    """Runs one schedule; "ok" or "deadlock" (asserts on early reuse)."""
+def simulate(rows, mode, na, seed, ncw=8, new=8, stall=False, early_release=False, mma_unplans=True,
+             slow=None):
+    """Runs one schedule; "ok" or "deadlock" (asserts on early reuse).
+
+    `slow` names a warp that is scheduled far less often than the others;
+    `mma_unplans=False` leaves the MMA warp out of a plan half's readers."""
     rng = random.Random(seed)
     mstep, pred = mode == "M", mode == "P"
     copies = 0 if mstep else NCOPY
     ngrp = new // 4
-    pfull, pempty = [Bar(1), Bar(1)], [Bar(ncw + new + copies) for _ in range(2)]
+    pfull, pempty = [Bar(1), Bar(1)], [Bar(ncw + new + copies + mma_unplans) for _ in range(2)]
     mfull, mempty = [Bar(32) for _ in range(NS)], [Bar(ncw + new) for _ in range(NS)]
     bfull, bempty = [Bar(NCOPY), Bar(NCOPY)], [Bar(1), Bar(1)]
     mma_done, conv = [Bar(1), Bar(1)], [Bar(ncw + (0 if mstep else 4)) for _ in range(2)]
@@ -89,7 +93,7 @@ def simulate(rows, mode, na, seed, ncw=8, new=8, stall=False, early_release=Fals
                     break
                 r, first, last = tiles[t]
                 plan[t % (2 * HALF)] = dict(t=t, n=r, row=r, first=first, last=last)
-                plan_users[t] = set(warps) | {("w", c) for c in range(copies)}
+                plan_users[t] = set(warps) | ({"mma"} if mma_unplans else set()) | {("w", c) for c in range(copies)}
             pfull[h & 1].arrive()
             if stop:
                 return
@@ -162,6 +166,8 @@ def simulate(rows, mode, na, seed, ncw=8, new=8, stall=False, early_release=Fals
             m, s = entry(t), t & 1
             if m["n"] < 0:
                 return
+            if mma_unplans:
+                unplan(t, "mma")
             row = m["row"]
             if m["first"]:
                 if not mstep:
@@ -261,7 +267,7 @@ def simulate(rows, mode, na, seed, ncw=8, new=8, stall=False, early_release=Fals
         order = list(range(len(actors)))
         rng.shuffle(order)
         for a in order:
-            if not alive[a] or rng.random() < 0.3:
+            if not alive[a] or rng.random() < (0.97 if a == {"mma": 1}.get(slow) else 0.3):
                 continue
             if waiting[a] is not None:
                 if not waiting[a][1].ready(waiting[a][2]):
@@ -296,6 +302,30 @@ def test_random_schedules_finish_without_early_reuse(mode, na, ncw, new):
         if seed % 10 == 0:
             rows = [rng.choice([1, 1, 2, 40]) for _ in range(25)]  # several plan halves
         assert simulate(rows, mode, na, seed, ncw, new) == "ok", (mode, seed, rows)
+
+
+# rows of several tiles, so that plan halves end inside a row, on many halves
+LONG_ROWS = [[3] * 120, [2, 1] * 120, [5] * 80, [40, 1, 30, 2, 61, 3, 70, 20, 90]]
+
+
+@pytest.mark.parametrize("mode,na,ncw,new", [("M", 2, 8, 8), ("M", 1, 4, 4), ("E", 2, 8, 8), ("P", 2, 8, 4)])
+@pytest.mark.parametrize("rows", range(len(LONG_ROWS)))
+def test_a_slow_mma_warp_reads_its_plan_entries(mode, na, ncw, new, rows):
+    for seed in range(4):
+        assert simulate(LONG_ROWS[rows], mode, na, seed, ncw, new, slow="mma") == "ok"
+
+
+def test_the_model_sees_a_plan_half_reused_under_the_mma_warp():
+    """The M-step's converters and epilogue can be done with a half whose last
+    tile does not end its row before the MMA warp has read that tile's entry."""
+    bad = 0
+    for seed in range(4):
+        for rows in LONG_ROWS:
+            try:
+                bad += simulate(rows, "M", 2, seed, 8, 8, slow="mma", mma_unplans=False) != "ok"
+            except AssertionError:
+                bad += 1
+    assert bad
 
 
 def test_a_copy_that_never_completes_blocks_the_mmas():
