@@ -111,32 +111,6 @@ __device__ __forceinline__ T quad_tri(const T *__restrict__ sU, const T (&delta)
   return q;
 }
 
-// Same quad form, also returning z = U^T delta (for gradients).
-template <typename T, int DP>
-__device__ __forceinline__ T quad_tri_z(const T *__restrict__ sU, const T (&delta)[DP], T (&z)[DP]) {
-  constexpr int V = Tri<T>::V;
-  using VT = typename Vec<T>::type;
-  T q = T(0);
-  int off = 0;
-#pragma unroll
-  for (int i = 0; i < DP; ++i) {
-    T y = T(0);
-#pragma unroll
-    for (int j = 0; j <= i; j += V) {
-      VT u = *reinterpret_cast<const VT *>(sU + off + j);
-      const T *uu = reinterpret_cast<const T *>(&u);
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        if (j + v <= i) y = fma(uu[v], delta[j + v], y);
-      }
-    }
-    z[i] = y;
-    q = fma(y, y, q);
-    off += Tri<T>::col_len(i);
-  }
-  return q;
-}
-
 // Cooperative copy of W_triu[n] (upper triangle of a [D,D] block with the
 // given row / column strides) into the packed layout, zero padded to DP.
 // Consecutive threads read consecutive columns of one row.
