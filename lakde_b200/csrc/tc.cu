@@ -1193,8 +1193,10 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
       for (int gr = 0; gr < NGRP; ++gr) m = fmaxf(m, part[gr * QB + e].x);
 #pragma unroll
       for (int gr = 0; gr < NGRP; ++gr) {
+        // (an untouched entry's sum is 0; (-inf, NaN) is one that has met only NaN
+        // terms: its NaN is kept whatever the other kernels gave)
         const float2 a = part[gr * QB + e];
-        if (a.x != -INFINITY) ssum += a.y * __expf(a.x - m);
+        if (a.y != 0.f) ssum += a.y * __expf(a.x - m);
       }
       const int64_t o = (int64_t)(blockIdx.x / g.nqb) * g.Nq + q0 + e;
       g.ws_m[o] = m;
