@@ -137,7 +137,8 @@ __device__ __forceinline__ void load_tri(T *__restrict__ sU, const T *__restrict
 // the low 13 bits zero): add half of the dropped range to the magnitude bits
 // and clear them.  Two integer ALU operations; finite inputs far below
 // FLT_MAX (centred differences and inverse factors) cannot carry into the
-// exponent's all-ones pattern.
+// exponent's all-ones pattern.  A NaN with the high payload bits set (as device
+// arithmetic gives it) becomes a zero: callers that may meet one look for it.
 __device__ __forceinline__ float tf32_rna(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
