@@ -65,14 +65,14 @@ def compute_knn_graph(X, k, bsize=1024, return_dists=False, include_self=False, 
     left = torch.cat((-2.0 * Xd, Xd.new_ones(N, 1)), 1)
     # at least 2 GB of distances a block (enough rows for the selection, a warp
     # each, to fill the GPU), bsize rows when those are more
-    bsize = min(N, max(bsize, 2**28 // N))
-    d = Xd.new_empty(bsize, N)
+    rows = max(bsize, 2**28 // max(N, 1))
+    d = Xd.new_empty(min(rows, N), N)
     I = torch.empty(N, k, dtype=dtype, device=X.device)
     Dout = X.new_empty(N, k) if return_dists else None
-    for i in range(0, N, bsize):
-        db = torch.mm(left[i : i + bsize], right, out=d[: N - i])
-        kernels.knn_select(db, Xd, i, k, include_self=include_self, out_idx=I[i : i + bsize],
-                           out_dist=None if Dout is None else Dout[i : i + bsize])
+    for i in range(0, N, rows):
+        db = torch.mm(left[i : i + rows], right, out=d[: N - i])
+        kernels.knn_select(db, Xd, i, k, include_self=include_self, out_idx=I[i : i + rows],
+                           out_dist=None if Dout is None else Dout[i : i + rows])
     if return_dists:
         return Dout, I
     return I

@@ -1,0 +1,50 @@
+"""Calls of compute_knn_graph that do not depend on a GPU's arithmetic, with
+the selection kernel replaced by a sort on the CPU."""
+
+import pytest
+import torch
+
+from lakde_b200 import utils
+
+
+@pytest.fixture
+def blocks(monkeypatch):
+    """The (rows, columns) of every distance block handed to the selection."""
+    seen = []
+
+    def select(dist, X, row0, k, include_self=False, out_idx=None, out_dist=None):
+        assert not dist.requires_grad
+        nb, N = dist.shape
+        seen.append((nb, N))
+        e = (X[row0 : row0 + nb, None] - X[None]).square().sum(2)
+        # the block orders the points as the distances do
+        assert torch.equal(dist.argsort(1, stable=True), e.argsort(1, stable=True))
+        if not include_self:
+            e[torch.arange(nb), torch.arange(nb) + row0] = torch.inf
+        d, i = e.sort(1, stable=True)
+        out_idx.copy_(i[:, :k])
+        if out_dist is not None:
+            out_dist.copy_(d[:, :k].sqrt())
+        return out_idx
+
+    monkeypatch.setattr(utils.kernels, "knn_select", select)
+    return seen
+
+
+def _points(N, D, seed=0):
+    return torch.randn(N, D, generator=torch.Generator().manual_seed(seed), dtype=torch.float64)
+
+
+def _exact(X, k):
+    e = (X[:, None] - X[None]).square().sum(2)
+    e.fill_diagonal_(torch.inf)
+    d, i = e.sort(1, stable=True)
+    return d[:, :k].sqrt(), i[:, :k]
+
+
+def test_no_points(blocks):
+    I = utils.compute_knn_graph(torch.empty(0, 5), 3)
+    assert I.shape == (0, 3) and I.dtype == torch.int32
+    d, I = utils.compute_knn_graph(torch.empty(0, 5), 3, return_dists=True)
+    assert d.shape == I.shape == (0, 3)
+    assert blocks == []
