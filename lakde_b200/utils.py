@@ -60,7 +60,7 @@ def compute_knn_graph(X, k, bsize=1024, return_dists=False, include_self=False, 
     if metric.lower() != "l2":
         raise ValueError("only the l2 metric is supported")
     N = X.size(0)
-    Xd = X.double().contiguous()
+    Xd = X.detach().double().contiguous()
     right = torch.cat((Xd, (Xd * Xd).sum(1, keepdim=True)), 1).T
     left = torch.cat((-2.0 * Xd, Xd.new_ones(N, 1)), 1)
     # at least 2 GB of distances a block (enough rows for the selection, a warp

@@ -48,3 +48,12 @@ def test_no_points(blocks):
     d, I = utils.compute_knn_graph(torch.empty(0, 5), 3, return_dists=True)
     assert d.shape == I.shape == (0, 3)
     assert blocks == []
+
+
+def test_points_that_require_grad(blocks):
+    X = _points(60, 4).requires_grad_()
+    d, I = utils.compute_knn_graph(X, 7, return_dists=True)
+    ed, ei = _exact(X.detach(), 7)
+    assert torch.equal(I.long(), ei)
+    torch.testing.assert_close(d, ed)
+    assert not d.requires_grad
