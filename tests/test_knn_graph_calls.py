@@ -18,10 +18,10 @@ def blocks(monkeypatch):
         seen.append((nb, N))
         e = (X[row0 : row0 + nb, None] - X[None]).square().sum(2)
         # the block orders the points as the distances do
-        assert torch.equal(dist.argsort(1, stable=True), e.argsort(1, stable=True))
+        assert torch.equal(dist.argsort(dim=1, stable=True), e.argsort(dim=1, stable=True))
         if not include_self:
             e[torch.arange(nb), torch.arange(nb) + row0] = torch.inf
-        d, i = e.sort(1, stable=True)
+        d, i = e.sort(dim=1, stable=True)
         out_idx.copy_(i[:, :k])
         if out_dist is not None:
             out_dist.copy_(d[:, :k].sqrt())
@@ -38,7 +38,7 @@ def _points(N, D, seed=0):
 def _exact(X, k):
     e = (X[:, None] - X[None]).square().sum(2)
     e.fill_diagonal_(torch.inf)
-    d, i = e.sort(1, stable=True)
+    d, i = e.sort(dim=1, stable=True)
     return d[:, :k].sqrt(), i[:, :k]
 
 
