@@ -56,16 +56,21 @@ def compute_knn_graph(X, k, bsize=1024, return_dists=False, include_self=False, 
     lakde_knn_select (kernels.knn_select) keeps each row's k + 8 smallest in one
     pass, re-ranks them by exact float64 differences and writes the k nearest,
     equal distances ordered by index.
+
+    ``bsize`` is the number of rows of distances held at once when it is below
+    the default; from the default on, a block takes at least that many rows and
+    as many as fit 2 GB.
     """
     if metric.lower() != "l2":
         raise ValueError("only the l2 metric is supported")
+    if bsize < 1:
+        raise ValueError("bsize must be positive")
     N = X.size(0)
     Xd = X.detach().double().contiguous()
     right = torch.cat((Xd, (Xd * Xd).sum(1, keepdim=True)), 1).T
     left = torch.cat((-2.0 * Xd, Xd.new_ones(N, 1)), 1)
-    # at least 2 GB of distances a block (enough rows for the selection, a warp
-    # each, to fill the GPU), bsize rows when those are more
-    rows = max(bsize, 2**28 // max(N, 1))
+    # 2 GB of distances: enough rows for the selection, a warp each, to fill the GPU
+    rows = bsize if bsize < 1024 else max(bsize, 2**28 // max(N, 1))
     d = Xd.new_empty(min(rows, N), N)
     I = torch.empty(N, k, dtype=dtype, device=X.device)
     Dout = X.new_empty(N, k) if return_dists else None

@@ -57,3 +57,25 @@ def test_points_that_require_grad(blocks):
     assert torch.equal(I.long(), ei)
     torch.testing.assert_close(d, ed)
     assert not d.requires_grad
+
+
+@pytest.mark.parametrize("bsize,sizes", [(16, [16, 16, 16, 2]), (50, [50]), (77, [50]), (1024, [50])])
+def test_a_small_block_size_bounds_the_block(blocks, bsize, sizes):
+    """Below the default, bsize is the number of rows of distances held at once."""
+    X = _points(50, 3)
+    assert torch.equal(utils.compute_knn_graph(X, 5, bsize=bsize).long(), _exact(X, 5)[1])
+    assert blocks == [(nb, 50) for nb in sizes]
+
+
+def test_the_default_block_grows_to_two_gigabytes(blocks, monkeypatch):
+    X = _points(1500, 2)
+    utils.compute_knn_graph(X, 5)
+    utils.compute_knn_graph(X, 5, bsize=1400)
+    utils.compute_knn_graph(X, 5, bsize=1023)
+    assert blocks == [(1500, 1500), (1500, 1500), (1023, 1500), (477, 1500)]
+
+
+@pytest.mark.parametrize("bsize", [0, -1])
+def test_block_size_must_be_positive(blocks, bsize):
+    with pytest.raises(ValueError):
+        utils.compute_knn_graph(_points(20, 2), 3, bsize=bsize)
