@@ -61,33 +61,36 @@ __device__ __forceinline__ constexpr int tix(int i, int j) { return i * (i + 1) 
 // rows are DP * 4 or DP * 8 bytes apart and start 16-byte aligned (DP in
 // {4, 8}) or 8-byte aligned (DP = 2): vector loads, so a gather of one row per
 // thread is one or two load instructions instead of DP.
-// FIXED: the address is the same on every turn of a loop around the call.
-template <typename T, int DP, bool FIXED = false>
+// m is a row of X for every thread, also one with nothing to do (row 0 then).
+// WIDE off (the prior's rows): no 256-bit loads, which the plain ones beat where
+// few rows are in flight.
+template <typename T, int DP, bool WIDE = true>
 __device__ __forceinline__ void load_row(const T *__restrict__ X, int64_t m, int D, T (&out)[DP]) {
   const uintptr_t base = reinterpret_cast<uintptr_t>(X);
   // rows of 32 bytes (or 64) from a 32-byte aligned base: one 256-bit load
   // per 32 bytes, so a warp's gather of scattered rows touches each row's
-  // line once instead of once per 16 bytes.  Not for an
-  // address that a loop does not change: the compiler may take the load, an
-  // asm statement, out of that loop and so past the alignment test
-  if constexpr (sizeof(T) * DP >= 32 && !FIXED) {
-    if (D == DP && (base & 31u) == 0) {
+  // line once instead of once per 16 bytes.  The compiler may move an asm
+  // statement past a test around it, so the load carries the alignment test as
+  // its own predicate
+  if constexpr (sizeof(T) * DP >= 32 && WIDE) {
+    const bool wide = D == DP && (base & 31u) == 0;
 #pragma unroll
-      for (int v = 0; v < (int)(sizeof(T) * DP / 32); ++v) {
-        const T *p = X + m * DP + v * (32 / (int)sizeof(T));
-        if constexpr (sizeof(T) == 4) {
-          asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                       : "=f"(out[8 * v]), "=f"(out[8 * v + 1]), "=f"(out[8 * v + 2]), "=f"(out[8 * v + 3]),
-                         "=f"(out[8 * v + 4]), "=f"(out[8 * v + 5]), "=f"(out[8 * v + 6]), "=f"(out[8 * v + 7])
-                       : "l"(p));
-        } else {
-          asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-                       : "=d"(out[4 * v]), "=d"(out[4 * v + 1]), "=d"(out[4 * v + 2]), "=d"(out[4 * v + 3])
-                       : "l"(p));
-        }
+    for (int v = 0; v < (int)(sizeof(T) * DP / 32); ++v) {
+      const T *p = X + m * DP + v * (32 / (int)sizeof(T));
+      if constexpr (sizeof(T) == 4) {
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %9, 0;\n\t"
+            "@q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+            : "=f"(out[8 * v]), "=f"(out[8 * v + 1]), "=f"(out[8 * v + 2]), "=f"(out[8 * v + 3]),
+              "=f"(out[8 * v + 4]), "=f"(out[8 * v + 5]), "=f"(out[8 * v + 6]), "=f"(out[8 * v + 7])
+            : "l"(p), "r"((int)wide));
+      } else {
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+            "@q ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];\n\t}"
+            : "=d"(out[4 * v]), "=d"(out[4 * v + 1]), "=d"(out[4 * v + 2]), "=d"(out[4 * v + 3])
+            : "l"(p), "r"((int)wide));
       }
-      return;
     }
+    if (wide) return;
   }
   if constexpr (sizeof(T) == 4 && DP >= 4) {
     if (D == DP && (base & 15u) == 0) {
@@ -130,7 +133,7 @@ __device__ __forceinline__ bool chol_rows(F &&S, const T *__restrict__ P, T scal
 #pragma unroll
   for (int i = 0; i < DP; ++i) {
     T row[DP];
-    if (P) load_row<T, DP, true>(P, i < D ? i : 0, D, row);
+    if (P) load_row<T, DP, false>(P, i < D ? i : 0, D, row);
 #pragma unroll
     for (int j = 0; j <= i; ++j) {
       double v;
@@ -235,14 +238,14 @@ template <typename T, int DP>
 __global__ void __launch_bounds__(128, (sizeof(T) == 4 && DP == 8) ? 3 : 1) vi_rows_kernel(RowArgs<T> g) {
   constexpr int TT = DP * (DP + 1) / 2;
   const int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (it >= g.N) return;
-  const int64_t n = g.order ? (int64_t)g.order[it] : it;
+  const bool own = it < g.N;
+  const int64_t n = !own ? 0 : g.order ? (int64_t)g.order[it] : it;
   const int D = g.D;
-  const int64_t start = g.rowptr[n], end = g.rowptr[n + 1];
-  bool bad = end < start;
-
   T xn[DP];
   load_row<T, DP>(g.X, n + g.koff, D, xn);
+  if (!own) return;
+  const int64_t start = g.rowptr[n], end = g.rowptr[n + 1];
+  bool bad = end < start;
 
   // ---------------------------------------------------------------- M-step
   // pairs in batches of U: the indices, then the point rows of a batch are
