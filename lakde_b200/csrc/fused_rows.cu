@@ -631,7 +631,9 @@ extern "C" int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts, cons
         vi_rows_kernel<TT, 8><<<blocks, 128, 0, as_stream(stream)>>>(g);
       return check_launch("vi_rows");
     }
-    // Rows a warp and lanes a row, by the number of rows.  One warp's chain
+    // Rows a warp and lanes a row, by the number of points, which every shard of a
+    // set shares: the lanes set the order of a row's sums, so a shard gives the
+    // rows of the full launch (N = npts) bit for bit.  One warp's chain
     // (index and point loads of each pass, the FP64 posterior) takes the same
     // time with 2 rows as with 32, so rows are packed only as far as the chip is
     // full without: 2, 4, 8, 16 and 32 rows a warp cross at 1,500 to 4,500
@@ -658,9 +660,10 @@ extern "C" int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts, cons
       return check_launch("vi_rows");
     };
     using std::integral_constant;
-    if (N <= 3000) return launch(integral_constant<int, 16>{}, integral_constant<int, 2>{});
-    if (N <= 8000) return launch(integral_constant<int, 8>{}, integral_constant<int, 4>{});
-    if (N <= 24000) return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{});
+    if (npts <= 3000) return launch(integral_constant<int, 16>{}, integral_constant<int, 2>{});
+    if (npts <= 8000) return launch(integral_constant<int, 8>{}, integral_constant<int, 4>{});
+    if (npts <= 24000) return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{});
+    // (the same two lanes: here the launch's own rows decide)
     if (N <= 72000) return launch(integral_constant<int, 2>{}, integral_constant<int, 16>{});
     return launch(integral_constant<int, 2>{}, integral_constant<int, 32>{});
   });
