@@ -724,14 +724,16 @@ __global__ void __launch_bounds__(32 * DmmaCfg<DP, LEAN>::WPB, DmmaCfg<DP, LEAN>
 }
 
 // failed = min(failed, min_n info_n): one pass with an atomic only where a
-// status is negative (a reduction and a minimum as two launches took 4 of an
+// status is below the value there (a reduction and a minimum as two launches took 4 of an
 // iteration's 26 us at 2,000 rows).
 __global__ void __launch_bounds__(256) fold_info_kernel(const int32_t *__restrict__ info, int64_t N,
                                                         int32_t *__restrict__ failed) {
-  int32_t worst = 0;
+  int32_t worst = 0x7fffffff;
+  // (read beside the statuses: another block's atomic only makes it lower)
+  const int32_t now = *failed;
   for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x)
     worst = min(worst, info[n]);
-  if (worst < 0) atomicMin(failed, worst);
+  if (worst < now) atomicMin(failed, worst);
 }
 
 }  // namespace lakde
