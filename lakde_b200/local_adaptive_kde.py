@@ -157,16 +157,23 @@ class LocallyAdaptiveKDE(VIModel, ABC):
         finfo = torch.finfo(X.dtype)
         coeff = torch.clamp_(torch.exp(self.rnm_log_consts - rnm_log_consts), min=finfo.tiny, max=finfo.max)
         sums = X.new_zeros(N)
-        cols = [ind[1].long() for ind, _ in self.rnm_blocks]
-        for bi, (col, (_, values)) in enumerate(zip(cols, self.rnm_blocks)):
+
+        def columns(bi):
+            # as they are stored: no int64 copy of them (a graph of another type keeps its own)
+            col = self.rnm_blocks[bi][0][1]
+            return col if col.dtype in (torch.int32, torch.int64) else col.long()
+
+        for bi, (_, values) in enumerate(self.rnm_blocks):
+            col = columns(bi)
             if bi != block_idx:
-                values *= coeff[col]
-            sums.scatter_add_(0, col, values)
+                values *= coeff.index_select(0, col)
+            sums.index_add_(0, col, values)
+            del col
         sums = torch.clamp_min(sums, finfo.eps)
         rnm_log_consts += sums.log()
         coeff = torch.clamp_(torch.reciprocal(sums), min=finfo.tiny, max=finfo.max)
-        for col, (_, values) in zip(cols, self.rnm_blocks):
-            values *= coeff[col]
+        for bi, (_, values) in enumerate(self.rnm_blocks):
+            values *= coeff.index_select(0, columns(bi))
         return rnm_log_consts
 
     # ------------------------------------------------------------- fused path
