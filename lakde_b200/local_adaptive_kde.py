@@ -50,8 +50,13 @@ def calc_log_rho_block(X_test, X_train, nu, W_triu, logdet_W):
 # in float32.  A step over one block of points at a time is 25 launches and a
 # synchronisation each, however small the block: an iteration on 2,000 points
 # of 2 dimensions in blocks of 512 took 10.5 ms so and 5.5 ms with one step a
-# kernel block.  Tens of millions of entries fill the GPU; more would only hold
-# more memory.
+# kernel block.  Tens of millions of entries fill the GPU (20,000 points of 2
+# dimensions in blocks of 512: 186 ms with 2^22 entries, 172 with 2^23, 150 with
+# 2^25, 706 block by block); more would only hold more memory.  A slab's
+# transients are 4 bytes an entry and 44 per entry that is kept: the peak of that
+# fit is 97 MB (72 block by block), of 50,000 points in blocks of 2,048 0.62 GB
+# (0.25), and where most entries are kept less than block by block, whose parts
+# were joined and sorted (3,000 points of 21 dimensions: 54 MB, before 123).
 DENSE_ENTRIES = 1 << 25
 
 
