@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(sweep::THREADS, sweep::Cfg<T, DP>::OCC) quad_d
   const int64_t n_begin = (blockIdx.x / m_tiles) * chunk;
   const int64_t n_end = (n_begin + chunk < N) ? n_begin + chunk : N;
   auto count = [&](int64_t n0) { return (int)((n_end - n0) < C::KT ? (n_end - n0) : C::KT); };
-  sweep::clear_stages<T, DP>(st, tid);
+  sweep::clear_stages<T, C>(st, n_end - n_begin, tid);
   __syncthreads();
   sweep::stage_kernels<T, DP>(st, W, ws0, ws1, ws2, Xn, xns0, xns1, n_begin, count(n_begin), D, tid);
   sweep::cp_async_commit();
@@ -451,9 +451,17 @@ extern "C" int lakde_chol_quad_form(int dtype, const void *W_triu, const int64_t
       int st = set_smem(kern, C::smem);
       if (st) return st;
       // about six waves of resident CTAs: the last wave costs little, and a
-      // CTA still shares its points over its chunk
+      // CTA still shares its points over its chunk.  At least eight kernels a
+      // CTA while that leaves two CTAs an SM, else four: a CTA's set-up (its
+      // points, the first stage, the code's way into the instruction cache) takes
+      // as long as three to six kernels.  us, chunk as by the waves alone / 4 / 8 /
+      // 16: float32 512 x 4,096 (chunk 2) at d = 16 48 / 32 / 29 / 27, at d = 8 17 /
+      // 12 / 11 / 10; float64 64 x 2,000 (1) at d = 32 41 / 20 / 19 / 32, at d = 48
+      // 57 / 36 / 36 / 65; 1,000 x 1 (1) at d = 40 34 / 30 / 33 / 63.
       const int64_t m_tiles = (M + C::TILE - 1) / C::TILE;
-      const int64_t chunk = sweep::chunk_len(N, m_tiles, 148 * 6 * C::OCC, C::KT);
+      const int64_t least = m_tiles * ((N + 7) / 8) >= 2 * 148 ? 8 : 4;
+      int64_t chunk = sweep::chunk_len(N, m_tiles, 148 * 6 * C::OCC, C::KT);
+      chunk = chunk < least ? least : chunk;
       const int64_t tiles = m_tiles * ((N + chunk - 1) / chunk);
       if (tiles > 0x7fffffffLL) {
         set_error("chol_quad_form: problem too large (%lld tiles)", (long long)tiles);

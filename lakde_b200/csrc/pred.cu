@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(sweep::THREADS, sweep::Cfg<T, DP>::OCC) pred_p
       sweep::cp_async_elem(d + k * C::KS + C::S0 + 1, nu + n0 + k);
     }
   };
-  sweep::clear_stages<T, DP>(st, tid);
+  sweep::clear_stages<T, C>(st, n_end - n_begin, tid);
   __syncthreads();
   stage(0, n_begin);
   sweep::cp_async_commit();

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(sweep::THREADS, BwdCfg<T, DP>::OCC) pred_bwd_p
       sweep::cp_async_elem(d + k * L::KS + L::S0 + 1, nu + n0 + k);
     }
   };
-  for (int e = tid; e < 2 * C::KT * L::KS; e += sweep::THREADS) st[e] = T(0);
+  sweep::clear_stages<T, L, C::KT>(st, n_end - n_begin, tid);
   __syncthreads();
   stage(0, n_begin);
   sweep::cp_async_commit();

@@ -315,11 +315,18 @@ struct Points {
   }
 };
 
-// Zeroes both stages once: their padding is never written again.
-template <typename T, int DP>
-__device__ __forceinline__ void clear_stages(T *st, int tid) {
-  using C = Cfg<T, DP>;
-  for (int e = tid; e < 2 * C::KT * C::KS; e += THREADS) st[e] = T(0);
+// Zeroes what a chunk of `kernels` will stage of both stages once: the padding
+// is never written again.
+template <typename T, typename C, int KT = C::KT>
+__device__ __forceinline__ void clear_stages(T *st, int64_t kernels, int tid) {
+  static_assert(C::KS % C::V == 0, "whole 16-byte vectors");
+  const int end = (int)(kernels < 2 * KT ? kernels : 2 * KT) * C::KS;
+  using VT = typename Vec<T>::type;
+  VT zero;
+  T *z = reinterpret_cast<T *>(&zero);
+#pragma unroll
+  for (int k = 0; k < C::V; ++k) z[k] = T(0);
+  for (int e = tid * C::V; e < end; e += THREADS * C::V) *reinterpret_cast<VT *>(st + e) = zero;
 }
 
 // Kernels per CTA so that tiles x chunks is about `ctas`; whole groups of kt
