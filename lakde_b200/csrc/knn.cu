@@ -4,10 +4,11 @@
 // turns each row of the block into that point's k nearest neighbours, nearest
 // first, equal distances ordered by index:
 //
-//   1. one CTA (small k: one warp) per row streams the row once, keeping every value below a
-//      running threshold in a shared-memory buffer; when the next chunk could
-//      overflow the buffer it is sorted (bitonic, by value then index) and cut
-//      to its kc = k + 8 smallest, whose largest becomes the threshold;
+//   1. one CTA (small k and many rows: one warp) per row streams the row once,
+//      keeping every value below a running threshold in a shared-memory buffer;
+//      when the next chunk could overflow the buffer it is sorted (bitonic, by
+//      value then index) and cut to its kc = k + 8 smallest, whose largest becomes
+//      the threshold;
 //   2. the kc candidates are re-ranked by exact float64 differences
 //      sum_d (x_c - x_r)^2 (the GEMM form cancels for close points) and the
 //      first k by (exact distance, index) are written.
@@ -389,9 +390,20 @@ extern "C" int lakde_knn_select(const void *dist, int64_t nb, int64_t N, int64_t
     using O = decltype(to);
     // a warp per row while 3/2 of its candidates and a step fit its buffer: 6 KB
     // up to 160 candidates (32 rows an SM in flight), 12 KB up to 500; beyond, a
-    // block per row, whose barriers cost less than a lone warp's sorts
-    if (kc <= 160) return launch_warps(ti, to, std::integral_constant<int, 512>{});
-    if (kc <= 500) return launch_warps(ti, to, std::integral_constant<int, 1024>{});
+    // block per row, whose barriers cost less than a lone warp's sorts.  And only
+    // with rows enough: below 8 warps an SM (1,184 rows) a launch takes as long as
+    // one warp over its row, 3.0 us per 1,000 values, while a block's threads share
+    // theirs; but a block also sorts its whole buffer, which short rows do not
+    // repay.  Block / warp, us, at 148, 592 and 1,024 rows: k = 5, 1,000,000 points
+    // 2245 / 3040, 2397 / 3074, 2655 / 3142; 400,000 points 955 / 1234, 1085 / 1248,
+    // 1240 / 1275; 100,000 points 305 / 327, 412 / 330, 505 / 336; 30,000 points 89 /
+    // 91, 215 / 111, 315 / 113; k = 490, 3,000 points 68 / 141, 193 / 141, 326 / 141;
+    // 400,000 points 1137 / 1441, 1490 / 1454, 2029 / 1480.
+    const bool many = nb > 8 * 148;
+    if (kc <= 160 && (many || N <= 32768 || (N <= 131072 && nb >= 256)))
+      return launch_warps(ti, to, std::integral_constant<int, 512>{});
+    if (kc > 160 && kc <= 500 && (many || (N <= 262144 && nb >= 600)))
+      return launch_warps(ti, to, std::integral_constant<int, 1024>{});
     auto kern = knn_select_kernel<I, O>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
       set_error("knn_select: cannot reserve %zu bytes of shared memory", smem);
