@@ -192,6 +192,12 @@ struct DmmaCfg {
   // spills: 0.308 and 0.179).  At 48 a cap of 168 gave 0.535 instead of 0.502 ms
   // for 30,000 matrices, and at 64 shared memory holds eight matrices anyway
   static constexpr int BLOCKS_PER_SM = LEAN ? 11 : DP <= 32 ? 8 : 1;
+  // ... and left free for no more matrices than 8 warps an SM take at once, each
+  // of which is then faster by itself: 1,000 matrices in float64 26.4 -> 22.8 us at
+  // d = 32, 15.8 -> 14.1 at d = 21, in float32 25.5 -> 23.6 at d = 32 (at 16 and
+  // below the capped form is as fast: 9.1 against 9.5 us for one matrix)
+  static constexpr bool FREE_FORM = !LEAN && DP > 16 && DP <= 32;
+  static constexpr int FREE_WARPS = 8;
   // per warp: FP64 tiles, 1 / L_ii, then the lower triangle of a per-matrix
   // FP32 T_n (packed rows or tiles, in doubles rounded up to 16 bytes), which
   // doubles as the scratch tile of the L output (T_n is then not staged)
@@ -701,9 +707,8 @@ __device__ __forceinline__ void factor_one(const FactorArgs<T> &g, int64_t n, do
 
 // Persistent: each warp walks matrices n, n + stride, ... (a grid of exactly
 // the resident blocks).
-template <typename T, int DP, bool LEAN>
-__global__ void __launch_bounds__(32 * DmmaCfg<DP, LEAN>::WPB, DmmaCfg<DP, LEAN>::BLOCKS_PER_SM)
-    factor_dmma_kernel(FactorArgs<T> g) {
+template <typename T, int DP, bool LEAN, int BLOCKS>
+__global__ void __launch_bounds__(32 * DmmaCfg<DP, LEAN>::WPB, BLOCKS) factor_dmma_kernel(FactorArgs<T> g) {
   using C = DmmaCfg<DP, LEAN>;
   extern __shared__ double smem_d[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -742,10 +747,10 @@ using namespace lakde;
 
 // Persistent DMMA launch: exactly the blocks that are resident at once
 // (registers and shared memory), so every block starts immediately.
-template <typename TT, int DP, bool LEAN>
+template <typename TT, int DP, bool LEAN, int BLOCKS = DmmaCfg<DP, LEAN>::BLOCKS_PER_SM>
 static int launch_factor_dmma_v(const FactorArgs<TT> &g, int64_t N, void *stream) {
   using C = DmmaCfg<DP, LEAN>;
-  auto kern = factor_dmma_kernel<TT, DP, LEAN>;
+  auto kern = factor_dmma_kernel<TT, DP, LEAN, BLOCKS>;
   if (C::smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
     if (e != cudaSuccess) {
@@ -775,6 +780,9 @@ template <typename TT, int DP>
 static int launch_factor_dmma(const FactorArgs<TT> &g, int64_t N, void *stream) {
   const bool lean_ok = !g.L && !g.Tm;
   if (lean_ok && tuning(LAKDE_TUNE_FACTOR, g.D) == 1) return launch_factor_dmma_v<TT, DP, true>(g, N, stream);
+  if constexpr (DmmaCfg<DP, false>::FREE_FORM) {
+    if (N <= DmmaCfg<DP, false>::FREE_WARPS * 148) return launch_factor_dmma_v<TT, DP, false, 1>(g, N, stream);
+  }
   return launch_factor_dmma_v<TT, DP, false>(g, N, stream);
 }
 
