@@ -67,8 +67,9 @@ LAKDE_API int lakde_max_dim(void);
  *                          that stage no T and write no L (else 0 is used).
  *   LAKDE_TUNE_ROWS:   0 = tensor-core rows from the caller's work queue;
  *                      1 = a static stride over the grid (the queue ignored).
- *   LAKDE_TUNE_VI_ROWS: 0 = lakde_vi_rows with a kernel row's pairs on two
- *                          lanes and its FP64 posterior on one lane per row;
+ *   LAKDE_TUNE_VI_ROWS: 0 = lakde_vi_rows with a kernel row's pairs on 16 to 2
+ *                          lanes, by the number of points, and its FP64
+ *                          posterior on one lane per row;
  *                      1 = one thread per kernel row.
  */
 typedef enum {
@@ -217,10 +218,11 @@ LAKDE_API int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts,
  * values, D <= 64.  The centred differences (x_m - x_n, and for the M-step
  * sqrt(r) (x_m - x_n)) and W_triu are split as x = hi + lo with
  * hi = tf32(x), lo = tf32(x - hi) (round to nearest); every product is
- * hi*hi + lo*hi + hi*lo with fp32 accumulation in tensor memory, within about
- * 2^-22 of the exact product (close to plain fp32 arithmetic).
+ * hi*hi + lo*hi + hi*lo + lo*lo with fp32 accumulation in tensor memory, within
+ * about 2^-22 of the exact product (close to plain fp32 arithmetic).  A NaN
+ * coordinate or factor makes what it takes part in NaN.
  *
- * Point rows are moved by bulk copies, so X (and Y) must have 16-byte
+ * Point rows are read by 16-byte loads, so X (and Y) must have 16-byte
  * aligned rows: base 16-byte aligned, row stride ldx (elements) a multiple
  * of 4 and >= D rounded up to 4; columns past D are never used.  Rows are
  * visited in `order` (may be NULL) through an atomic work queue: `queue`
@@ -492,7 +494,7 @@ LAKDE_API size_t lakde_log_pred_density_tc_workspace(int64_t N, int64_t Nq,
 
 /*
  * lakde_log_pred_density with the quad forms on the tensor cores (the tf32
- * hi / lo kernels above; queries in blocks of 2048, every query of a block
+ * hi / lo kernels above; queries in blocks of 256, every query of a block
  * against every kernel), float32 values, D <= 64, X [N, ldx] and Y [Nq, ldy]
  * with 16-byte aligned rows, W_triu given as W cores
  * (lakde/local_adaptive_kde.py:200-223).  *err as for the tensor-core E-step.

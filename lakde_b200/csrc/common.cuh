@@ -162,7 +162,8 @@ __device__ __forceinline__ double digamma_d(double x) {
 //   sum_{j < n} psi(x - j) = n psi(x) - sum_{k=1..n-1} (n - k) / (x - k):
 // two series and one division per step of both chains, instead of a series,
 // a logarithm and up to six recurrence divisions per term (at D = 63 the
-// E-step's row constants took 25k cycles per 32 rows of its metadata warp).
+// E-step's row constants took 25k cycles per 32 rows of the one warp that forms
+// them).
 __device__ __forceinline__ double mvdigamma_d(double a, int D) {
   if (!(a + 0.5 * (1 - D) > 0.0)) return nan("");
   const int n1 = (D + 1) / 2, n2 = D / 2;

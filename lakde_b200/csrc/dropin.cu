@@ -288,8 +288,8 @@ __global__ void scatter_cov_cta(const RP *__restrict__ rowptr, const CI *__restr
 // the gather from L2.  20,000 rows of 80 pairs on average at d = 43: 698 -> 259
 // us, the tensor pipe 46 % busy (a fifth of the time is the longest rows' tail);
 // d = 63 1278 -> 450, d = 24 2211 -> 121 (the CTA form above, whose 4 x 4
-// register blocks read both operands from shared memory; it stays for float32,
-// where the FP32 pipe has twice the rate: 417 us at d = 43).
+// register blocks read both operands from shared memory; it is still the
+// float32 form, 417 us at d = 43, and has not been tried against this one there).
 // ---------------------------------------------------------------------------
 template <typename RP, typename CI, int DP>
 __global__ void __launch_bounds__(32, DP <= 32 ? 16 : DP <= 48 ? 12 : 8)

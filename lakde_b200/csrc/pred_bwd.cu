@@ -27,6 +27,7 @@ struct BwdCfg : sweep::Cfg<T, DP, false> {
   static constexpr int P = sizeof(T) == 4 && DP <= 32 ? 2 : 1;
   static constexpr int TILE = sweep::THREADS * P;
   static constexpr int KT = DP <= 8 ? 16 : DP <= 32 ? 8 : 2;
+  // CTAs an SM is asked for (float64 at 64 dimensions: 135 KB leave one)
   static constexpr int OCC = DP <= 32 && sizeof(T) == 4 ? 3 : 2;
   // two stages, the queries, the warps' sums of g w
   static constexpr size_t smem =

@@ -46,8 +46,9 @@ struct Cfg {
   static constexpr int KT = ROLLED ? 1 : (DP <= 8 ? 32 : DP <= 16 ? 16 : 8);
   static constexpr size_t ybytes = ROLLED ? (size_t)DP * TILE * sizeof(T) : 0;
   static constexpr size_t smem = 2 * (size_t)KT * KS * sizeof(T) + ybytes;
-  // resident CTAs an SM is asked for (the registers then fit; shared memory
-  // sets the rolled form's two)
+  // resident CTAs an SM is asked for (the registers then fit).  The rolled form's
+  // two fit the shared memory but for float64 at 64 dimensions, whose 115,744
+  // bytes leave one (32 bytes too many), and the chunk rules count two there
   static constexpr int OCC = ROLLED ? 2 : sizeof(T) == 4 ? (DP <= 8 ? 4 : 3) : (DP <= 8 ? 4 : 3);
 
   // Element (j, i), j <= i, of the packed factor: row j from column V (j / V)

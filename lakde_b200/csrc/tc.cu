@@ -54,7 +54,7 @@
 // them back to convert, met at a named barrier per tile and all ran the
 // epilogue, and one warp planned tile by tile.  Measured, 50,000 rows, before ->
 // now, E-step: d = 63, 100 pairs a row 0.95 -> 0.55 ms, 30 pairs 0.87 -> 0.49;
-// d = 21, 64 pairs 0.54 -> 0.28; d = 13, 40 pairs 0.46 -> 0.19.  M-step: d = 63 0.91
+// d = 21, 64 pairs 0.54 -> 0.29; d = 13, 40 pairs 0.46 -> 0.19.  M-step: d = 63 0.91
 // -> 0.61 and 0.80 -> 0.46 ms, d = 21 0.69 -> 0.31, d = 13 0.67 -> 0.23.  Predictive
 // density, 5,000 kernels x 4,096 queries: d = 63 2.12 -> 1.24 ms, d = 43 1.76 -> 1.18,
 // d = 21 1.39 -> 0.68, d = 13 1.39 -> 0.48.
@@ -492,8 +492,8 @@ struct Kern {
   }
 
   // Writes them into slot ms, validated, and arrives on mfull (every lane).
-  // Brings a new row's W cores and kernel centre into L2: the slot is up to NS
-  // tiles ahead of the consumers.
+  // Brings a new row's W cores into L2: the slot is up to NS tiles ahead of the
+  // consumers.
   static __device__ __forceinline__ void write_tile(const Args &g, const Meta &m, const int32_t (&c)[4],
                                                     const float (&w)[4], unsigned char *sm, uint64_t *mfull, int ms,
                                                     int lane) {
@@ -1351,7 +1351,7 @@ int launch_rows(const char *what, tc::Args g, int64_t rows, void *stream) {
   if (grid > rows) grid = rows;
   if (grid < 1) grid = 1;
   // eight or more claims per CTA (the tail and small row counts balance), at
-  // most a row per lane of the metadata warp
+  // most a row per lane of the planner warp
   const int64_t batch = rows / (8 * grid);
   g.batch = (int)(batch < 1 ? 1 : batch > 32 ? 32 : batch);
   kern<<<(unsigned)grid, tc::Cfg<MODE, DP>::THREADS, smem, as_stream(stream)>>>(g);

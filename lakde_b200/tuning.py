@@ -4,8 +4,9 @@ Some kernels have more than one launch form that computes the same values
 (``lakde_tuning_set`` in include/lakde_b200.h): the FP64 factorisation with two
 warps per block or a lean form with one warp per block and 11 blocks per SM,
 the tensor-core kernels with their rows from an atomic work queue or on a
-static stride, the fused D <= 8 pass with a kernel row's pairs on two lanes
-(its FP64 posterior on one lane per row) or with one thread per kernel row.  Which is faster depends on D, N and the pair counts, so the
+static stride, the fused D <= 8 pass with a kernel row's pairs on 16 to 2 lanes
+by the number of points (named two_lanes_per_row; its FP64 posterior on one lane
+per row) or with one thread per kernel row.  Which is faster depends on D, N and the pair counts, so the
 fused engine times every choice on its own data before its first CUDA-graph
 capture and keeps the fastest, per knob and class of D (the library's table
 is process-wide).  The factorisation and row-schedule choices give identical
