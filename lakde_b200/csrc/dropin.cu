@@ -451,15 +451,17 @@ extern "C" int lakde_chol_quad_form(int dtype, const void *W_triu, const int64_t
       int st = set_smem(kern, C::smem);
       if (st) return st;
       // about six waves of resident CTAs: the last wave costs little, and a
-      // CTA still shares its points over its chunk.  At least eight kernels a
-      // CTA while that leaves two CTAs an SM, else four: a CTA's set-up (its
-      // points, the first stage, the code's way into the instruction cache) takes
-      // as long as three to six kernels.  us, chunk as by the waves alone / 4 / 8 /
+      // CTA still shares its points over its chunk.  Of more than two CTAs an SM
+      // at a kernel each, at least eight kernels a CTA while that leaves two
+      // CTAs an SM, else four: a CTA's set-up (its points, the first stage, the
+      // code's way into the instruction cache) takes as long as several kernels
+      // up to 48 dimensions.  us, chunk as by the waves alone / 4 / 8 /
       // 16: float32 512 x 4,096 (chunk 2) at d = 16 48 / 32 / 29 / 27, at d = 8 17 /
       // 12 / 11 / 10; float64 64 x 2,000 (1) at d = 32 41 / 20 / 19 / 32, at d = 48
-      // 57 / 36 / 36 / 65; 1,000 x 1 (1) at d = 40 34 / 30 / 33 / 63.
+      // 57 / 36 / 36 / 65; 1,000 x 1 (1) at d = 40 34 / 30 / 33 / 63; 34 x 336 (1) at
+      // d = 63 21 / 29.
       const int64_t m_tiles = (M + C::TILE - 1) / C::TILE;
-      const int64_t least = m_tiles * ((N + 7) / 8) >= 2 * 148 ? 8 : 4;
+      const int64_t least = m_tiles * N <= 2 * 148 ? 1 : m_tiles * ((N + 7) / 8) >= 2 * 148 ? 8 : 4;
       int64_t chunk = sweep::chunk_len(N, m_tiles, 148 * 6 * C::OCC, C::KT);
       chunk = chunk < least ? least : chunk;
       const int64_t tiles = m_tiles * ((N + chunk - 1) / chunk);
