@@ -14,6 +14,8 @@
 //      first k by (exact distance, index) are written.
 //
 // The point itself is excluded unless include_self (lakde/utils.py:104-105).
+// Values that are not finite are no distances (a row of a point with an infinite
+// coordinate holds -inf and +inf): such a row has neighbours -1.
 #include "common.cuh"
 
 namespace lakde {
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(kKnnThreadsLarge) knn_select_kernel(const doub
       if (j < N) {
         double v = drow[j];
         if (v != v || (!include_self && j == self)) v = inf;
-        if (v < t_now) {
+        if (v < t_now && v > -inf) {
           const int p = atomicAdd(&cnt, 1);
           key[p] = v;
           idx[p] = (int32_t)j;
@@ -293,9 +295,10 @@ __global__ void __launch_bounds__(32 * kWarpRows) knn_select_warp_kernel(const d
 #pragma unroll
     for (int e = 0; e < kWarpStep / 32; ++e) {
       const int64_t j = base + 64 * (e / 2) + 2 * lane + (e & 1);
-      const bool in = v[e] < thr && (include_self || j != self);  // false for NaN
+      bool in = v[e] < thr && (include_self || j != self);  // false for NaN
+      if (!__any_sync(0xffffffffu, in)) continue;
+      in = in && v[e] > -inf;
       const unsigned m = __ballot_sync(0xffffffffu, in);
-      if (m == 0) continue;
       if (in) {
         const int p = cnt + __popc(m & below);
         key[p] = v[e];
