@@ -55,9 +55,14 @@ __global__ void __launch_bounds__(32 * kGramWarps) gram_partial_kernel(const T *
     gram_load<T, NT>(W + n * DD, 0, D, lane, f[0]);
     wn = w[n];
   }
+  bool left = false;
   while (n < N) {
     const int64_t nn = n + stride;
     const double wd = (double)wn;
+    // a kernel of infinite weight is left for the end: times the zeros of a
+    // fragment its weight would make the whole sum NaN
+    const bool take = !isinf(wd);
+    left = left || !take;
 #pragma unroll
     for (int J = 0; J < NT; ++J) {
       // block J is in f[J % 2] (NT even: the next kernel's block 0 in f[0])
@@ -69,6 +74,7 @@ __global__ void __launch_bounds__(32 * kGramWarps) gram_partial_kernel(const T *
       }
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
+        if (!take) break;
         double b[NT];
 #pragma unroll
         for (int I = 0; I < NT; ++I)
@@ -101,12 +107,28 @@ __global__ void __launch_bounds__(32 * kGramWarps) gram_partial_kernel(const T *
     __syncthreads();
   }
   const int tri = D * (D + 1) / 2;
+  const bool infinite = __syncthreads_or(left);
   for (int e = threadIdx.x; e < NTILE * 64; e += 32 * kGramWarps) {
     int I = 0;
     const int t = e >> 6;
     while ((I + 1) * (I + 2) / 2 <= t) ++I;
     const int i = 8 * I + ((e >> 3) & 7), k = 8 * (t - I * (I + 1) / 2) + (e & 7);
-    if (i < D && k <= i) partials[(int64_t)blockIdx.x * tri + i * (i + 1) / 2 + k] = red[e];
+    if (i >= D || k > i) continue;
+    double sum = red[e];
+    if (infinite) {
+      // w times the finished element of W W^T
+#pragma unroll 1
+      for (int64_t m0 = (int64_t)blockIdx.x * kGramWarps; m0 < N; m0 += stride)
+#pragma unroll 1
+        for (int64_t m = m0; m < m0 + kGramWarps && m < N; ++m) {
+          if (!isinf((double)w[m])) continue;
+          double el = 0.0;
+#pragma unroll 1
+          for (int j = i; j < D; ++j) el = fma((double)W[m * DD + i * D + j], (double)W[m * DD + k * D + j], el);
+          sum = fma((double)w[m], el, sum);
+        }
+    }
+    partials[(int64_t)blockIdx.x * tri + i * (i + 1) / 2 + k] = sum;
   }
 }
 
