@@ -12,7 +12,7 @@
 // and then over the blocks, so the result does not depend on scheduling.
 //
 // Bound by the FP64 tensor pipe: NT (NT + 1) (NT + 2) / 3 MMAs of 16 cycles per
-// kernel.  20,000 kernels at d = 43: 350 + 64 -> 89 + 5 us (scalar FMAs on 4 x 4
+// kernel.  20,000 kernels at d = 43, both launches: 414 -> 72 us (scalar FMAs on 4 x 4
 // register blocks staged through shared memory, and one thread walking all
 // partials of an element, before).
 #include "common.cuh"
