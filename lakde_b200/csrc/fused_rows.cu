@@ -376,42 +376,32 @@ struct RowSlot {
 // neighbours, against 259 with B = 4, 299 at 12 warps with B = 4 (the former 168
 // registers) and 289 at 20 warps (spills).  Below DP = 8 the registers bind
 // nothing and B = 4 leads (2,000 rows of 2: 14.6 us at 32 rows a warp, 16.2
-// with B = 3); so it does where rows of 5 to 7 are padded to 8 and loaded
-// element-wise (WHOLE false: 100,000 rows of 5, K = 24 106 us, 111 with B = 3).
-template <typename T, int DP, bool WHOLE>
+// with B = 3).  Rows of 5 to 7, padded to 8, take the plan of 8: at 12 warps and
+// B = 4 d = 5, K = 16 takes 66 us instead of 61 at 72,000 rows and 73 instead of 77
+// at 85,000, where the 12 warps leave a wave less empty.
+template <typename T, int DP>
 struct RowPlan {
-  static constexpr bool WIDE = sizeof(T) == 4 && DP == 8 && WHOLE;
+  static constexpr bool WIDE = sizeof(T) == 4 && DP == 8;
   static constexpr int BLOCKS = WIDE ? 4 : 3;                    // of 128 threads an SM
   static constexpr int B = sizeof(T) == 8 ? 2 : WIDE ? 3 : 4;  // pairs in flight a lane
 };
 
-//
-// SHORT: two times RW rows a warp when the rows are short (at most kShortRow
-// pairs on average), which the first and last entry of rowptr tell: the FP64
-// posterior, a lane per row, is then most of a warp's work.  Changes no sum.
-constexpr int kShortRow = 32;
-
-template <typename T, int DP, bool WHOLE, int LPR, int RW, bool SHORT>
-__global__ void __launch_bounds__(128, RowPlan<T, DP, WHOLE>::BLOCKS) vi_rows_lanes_kernel(RowArgs<T> g) {
-  constexpr int B = RowPlan<T, DP, WHOLE>::B;
+template <typename T, int DP, int LPR, int RW>
+__global__ void __launch_bounds__(128, RowPlan<T, DP>::BLOCKS) vi_rows_lanes_kernel(RowArgs<T> g) {
+  constexpr int B = RowPlan<T, DP>::B;
   constexpr int TT = DP * (DP + 1) / 2;
-  constexpr int GROUPS = 32 / LPR, MOST = SHORT ? 2 * RW : RW;
-  static_assert(MOST <= 32, "a lane per row");
+  constexpr int GROUPS = 32 / LPR, PASSES = RW / GROUPS;
   constexpr unsigned FULL = 0xffffffffu;
   using RS = RowSlot<T, DP>;
-  __shared__ T park[4][MOST][RS::SIZE];
+  __shared__ T park[4][RW][RS::SIZE];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (LPR - 1), grp = lane / LPR;
-  int rw = RW;
-  if (SHORT && g.rowptr[g.N] - g.rowptr[0] <= kShortRow * g.N) rw = 2 * RW;
-  const int passes = rw / GROUPS;
-  const int64_t base = ((int64_t)blockIdx.x * 4 + warp) * rw;
-  if (SHORT && base >= g.N) return;
+  const int64_t base = ((int64_t)blockIdx.x * 4 + warp) * RW;
   T(*slot)[RS::SIZE] = park[warp];
   const int D = g.D;
   // each lane loads the setup of one of the warp's rows (row index, pair
   // range, its point row); the groups take their row's from that lane
   int64_t own_n = 0, own_start = 0, own_end = 0;
-  const bool own = lane < rw && base + lane < g.N;
+  const bool own = lane < RW && base + lane < g.N;
   if (own) {
     own_n = g.order ? (int64_t)g.order[base + lane] : base + lane;
     own_start = g.rowptr[own_n];
@@ -422,7 +412,7 @@ __global__ void __launch_bounds__(128, RowPlan<T, DP, WHOLE>::BLOCKS) vi_rows_la
 
   // ---------------------------------------------------------------- M-step
 #pragma unroll 1
-  for (int pass = 0; pass < passes; ++pass) {
+  for (int pass = 0; pass < PASSES; ++pass) {
     const int rl = pass * GROUPS + grp;
     const int64_t n = __shfl_sync(FULL, own_n, rl);
     const int64_t start = __shfl_sync(FULL, own_start, rl);
@@ -515,7 +505,7 @@ __global__ void __launch_bounds__(128, RowPlan<T, DP, WHOLE>::BLOCKS) vi_rows_la
   // ---------------------------------------------------------------- E-step
   const T nanv = T(NAN);
 #pragma unroll 1
-  for (int pass = 0; pass < passes; ++pass) {
+  for (int pass = 0; pass < PASSES; ++pass) {
     const int rl = pass * GROUPS + grp;
     const int64_t n = __shfl_sync(FULL, own_n, rl);
     const int64_t start = __shfl_sync(FULL, own_start, rl);
@@ -656,46 +646,39 @@ extern "C" int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts, cons
     // 231 / 136 / 90 / 73 / 111, 200,000 rows 1208 / 667 / 391 / 298 / 249;
     // float64 d = 8: 3,000 rows 29 / 34 / 46 / 73 / 126, 60,000 rows 458 / 275
     // / 185 / 145 / 183.
-    auto launch = [&](auto lpr, auto rw, auto by_length) {
+    auto launch = [&](auto lpr, auto rw) {
       constexpr int LPR = decltype(lpr)::value, RW = decltype(rw)::value;
-      constexpr bool SHORT = decltype(by_length)::value;
       const int64_t blocks = (N + 4 * RW - 1) / (4 * RW);
       if (blocks > 0x7fffffffLL) {
         set_error("vi_rows: too many rows");
         return (int)LAKDE_EUNSUPPORTED;
       }
       if (D <= 2)
-        vi_rows_lanes_kernel<TT, 2, true, LPR, RW, SHORT><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+        vi_rows_lanes_kernel<TT, 2, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
       else if (D <= 4)
-        vi_rows_lanes_kernel<TT, 4, true, LPR, RW, SHORT><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
-      else if (D == 8 || sizeof(TT) == 8)  // (one plan in float64)
-        vi_rows_lanes_kernel<TT, 8, true, LPR, RW, SHORT><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+        vi_rows_lanes_kernel<TT, 4, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
       else
-        vi_rows_lanes_kernel<TT, 8, sizeof(TT) == 8, LPR, RW, SHORT>
-            <<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
+        vi_rows_lanes_kernel<TT, 8, LPR, RW><<<(unsigned)blocks, 128, 0, as_stream(stream)>>>(g);
       return check_launch("vi_rows");
     };
     using std::integral_constant;
-    // The twice as wide packing that a set of short rows takes (SHORT) costs the
-    // launch two loads before its first, a tenth at three to seven dimensions, so it
-    // is kept to where it gains more, and to more rows than are resident at once.
-    // us with the fewer / the more rows a warp, float32: d = 8, 48,000 points, K = 10
-    // 58 / 51, d = 5, 23,500, K = 10 44 / 33; float64: d = 8, 60,000, K = 16 93 / 76.
-    using std::false_type;
-    using std::true_type;
+    // That was measured on long rows; with few pairs a row the posterior, a lane
+    // per row, is most of a warp's work and full warps lead earlier, so the bounds
+    // are drawn where neither loses much on kNN patterns.  us at K = 10 / 16 / 24 / 50,
+    // 16 / 32 rows a warp, float32: d = 5, 48,000 points 52 61 70 90 / 41 51 64 110,
+    // 40,000 47 51 57 76 / 41 50 64 106; d = 8, 72,000 61 67 75 99 / 53 65 80 131; d = 4,
+    // 48,000 24 27 29 46 / 21 26 34 58, 56,000 26 33 39 52 / 21 26 33 59; float64 d = 8,
+    // 56,000 65 75 88 132 / 61 76 101 178, 64,000 91 104 118 167 / 71 78 104 185.  And
+    // 8 rows of 4 lanes / 16 of 2: float32 d = 8, 17,500 29 31 35 47 / 30 33 40 63,
+    // 20,000 46 48 52 54 / 32 37 43 66.
     constexpr bool F32 = sizeof(TT) == 4;
-    if (npts <= 3000) return launch(integral_constant<int, 16>{}, integral_constant<int, 2>{}, false_type{});
-    if (npts <= 8000) return launch(integral_constant<int, 8>{}, integral_constant<int, 4>{}, false_type{});
-    if (npts <= 24000) {
-      if (F32 && D > 4 && N > 17000)
-        return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{}, true_type{});
-      return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{}, false_type{});
-    }
+    if (npts <= 3000) return launch(integral_constant<int, 16>{}, integral_constant<int, 2>{});
+    if (npts <= 8000) return launch(integral_constant<int, 8>{}, integral_constant<int, 4>{});
+    if (npts <= (F32 && D > 4 ? 18000 : 24000))
+      return launch(integral_constant<int, 4>{}, integral_constant<int, 8>{});
     // (the same two lanes from here on: the launch's own rows decide)
-    if (N <= (D <= 2 ? 72000 : D <= 4 ? (F32 ? 50000 : 72000) : 40000))
-      return launch(integral_constant<int, 2>{}, integral_constant<int, 16>{}, false_type{});
-    if ((D == 8 || (!F32 && D > 4)) && N <= 72000)
-      return launch(integral_constant<int, 2>{}, integral_constant<int, 16>{}, true_type{});
-    return launch(integral_constant<int, 2>{}, integral_constant<int, 32>{}, false_type{});
+    const int64_t bound = D <= 2 ? 72000 : D <= 4 ? (F32 ? 50000 : 72000) : F32 ? (D == 8 ? 72000 : 40000) : 56000;
+    if (N <= bound) return launch(integral_constant<int, 2>{}, integral_constant<int, 16>{});
+    return launch(integral_constant<int, 2>{}, integral_constant<int, 32>{});
   });
 }
