@@ -358,6 +358,12 @@ struct Kern {
     bool exhausted;   // no rows left to fetch (uniform)
   };
 
+  // Whether one of the D elements of a row is NaN, by the whole warp.
+  static __device__ __forceinline__ bool row_has_nan(const float *x, int D, int lane) {
+    const float u = lane < D ? x[lane] : 0.f, v = 32 + lane < D ? x[32 + lane] : 0.f;
+    return __any_sync(0xffffffffu, u != u || v != v);
+  }
+
   // The next row slots of this CTA: the work queue (an atomic counter over the
   // caller's row order, `batch` slots per claim), a static stride over the grid
   // without a queue (32 slots), or the CTA's contiguous chunk of kernels for
@@ -398,15 +404,19 @@ struct Kern {
         c1 = -0.5f * nv;
       } else if (MODE == PRED) {
         c0 = g.lc[n];
-        // a NaN centre, which the split would lose, makes the kernel's term NaN
-        const float *x = g.X + n * g.ldx;
-#pragma unroll 8
-        for (int d = 0; d < g.D; ++d)
-          if (x[d] != x[d]) c0 = NAN;
         c1 = 0.5f * (g.nu[n] + 1.f);
       }
     }
     const int got = __popc(__ballot_sync(0xffffffffu, valid));
+    if (MODE == PRED) {
+      // a NaN centre, which the split would lose, makes the kernel's term NaN (a
+      // row by all lanes: a lane per row took 2 us of a call on one query)
+#pragma unroll 4
+      for (int j = 0; j < got; ++j) {
+        const bool nan = row_has_nan(g.X + __shfl_sync(0xffffffffu, n, j) * g.ldx, g.D, lane);
+        if (nan && lane == j) c0 = NAN;
+      }
+    }
     if (got < (MODE != PRED && g.queue ? g.batch : 32)) P.exhausted = true;
     P.n = n;
     P.a = a;
@@ -585,7 +595,9 @@ struct Kern {
   // 0.342 -> 0.350 / 0.359 -> 0.363 (a clamp of the bits: 0.545 / 0.621, 0.351 /
   // 0.366; the conversion instruction: 3 % of a fit; one test per tile and a
   // second pass over it: 5 %, more code than the instruction cache holds).  The
-  // predictive density looks at its queries and centres outside its tile loop.
+  // predictive density looks at its centres and queries in the planner and
+  // epilogue warps, outside the tile loop (in the converters, which hold them, it
+  // cost 5 to 10 % at 48 dimensions; in the copy warps 15 % of ten queries).
   static __device__ __forceinline__ float rna_lo(float rest, uint32_t m) {
     if (MODE == PRED) return rna(rest, m);
     const float r = fmaf(rest, 0.f, __uint_as_float(__float_as_uint(rest) + 0x1000u));
@@ -953,6 +965,7 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
   };
   // predictive density: running (max, sum) of this thread's query in each query tile
   float2 run0 = make_float2(-INFINITY, 0.f), run1 = run0;
+  unsigned qnan = 0;  // and whether that query holds a NaN (bit per tile)
 
   if (warp == WARP_MMA) {
     // ----------------------------------------------------------- MMA warp
@@ -1093,15 +1106,7 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
 #pragma unroll
         for (int i = 0; i < NPQ; ++i) {
           const int64_t q = q0 + tl * MT + (i * Smem::NCW + warp) * Smem::RW + lane / Smem::LPR;
-          if (k < rch && q < g.Nq) {
-            // a query with a NaN has no density: as an infinity, which the split
-            // keeps, it has none either
-            const float4 v = ldg_row(g.Y + q * g.ldy + 4 * k);
-            const uint4 m = K::dim_masks(k, g.D);
-            y[tl][i] = v;
-            if (v.x != v.x || (m.y && v.y != v.y) || (m.z && v.z != v.z) || (m.w && v.w != v.w))
-              y[tl][i].x = INFINITY;
-          }
+          if (k < rch && q < g.Nq) y[tl][i] = ldg_row(g.Y + q * g.ldy + 4 * k);
         }
     }
     if (ok && K::meta_of(sm, 0).n >= 0) {
@@ -1158,6 +1163,17 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
     bool bad = false, ok = true;
     // the first two tiles have no earlier accumulator to wait for
     if (MODE != MSTEP && grp == 0 && lane < 2) mbar_arrive(conv + lane);
+    if (MODE == PRED) {
+      // queries of this warp's lanes with a NaN, which the split would lose
+      const int64_t q0 = (int64_t)(blockIdx.x % g.nqb) * QB + 32 * w4;
+#pragma unroll 1
+      for (int tl = 0; tl < 2; ++tl) {
+        const int64_t left = g.Nq - (q0 + tl * MT);
+#pragma unroll 4
+        for (int j = 0; j < (left < 32 ? (int)left : 32); ++j)
+          if (K::row_has_nan(g.Y + (q0 + tl * MT + j) * g.ldy, g.D, lane) && lane == j) qnan |= 1u << tl;
+      }
+    }
     for (int t = 0;; ++t) {
       ok = __all_sync(0xffffffffu, ready(t));
       if (!ok) break;
@@ -1210,8 +1226,9 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
     float2 *part = reinterpret_cast<float2 *>(sm + Smem::TILE);  // [NGRP][2][128], the A tiles are done
     if (warp >= WARP_EPI && warp < WARP_PLAN) {
       const int e = ((warp - WARP_EPI) >> 2) * QB + (warp & 3) * 32 + lane;
-      part[e] = run0;
-      part[e + MT] = run1;
+      // (a query with a NaN has no density, as in the plain kernel)
+      part[e] = qnan & 1u ? make_float2(-INFINITY, 0.f) : run0;
+      part[e + MT] = qnan & 2u ? make_float2(-INFINITY, 0.f) : run1;
     }
     __syncthreads();
     const int64_t q0 = (int64_t)(blockIdx.x % g.nqb) * QB;
