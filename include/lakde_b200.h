@@ -186,8 +186,8 @@ LAKDE_API int lakde_estep_logrho(int dtype, int64_t N, int64_t D, int64_t npts,
                        void *logrho, void *stream);
 
 /*
- * One VI iteration's per-kernel work for D <= 8 in a single pass, one thread
- * per kernel row (kernels are the points 0..N-1 of X[npts,D]):
+ * One VI iteration's per-kernel work for D <= 8 in a single pass (kernels are
+ * the points 0..N-1 of X[npts,D]; see LAKDE_TUNE_VI_ROWS for the forms):
  *   nu_n = nu_0 + sum_p r_p and S_n = sum_p r_p (x_m - x_n)(x_m - x_n)^T
  *   L_n = chol(nu_0 a_n / b_n P_n + S_n + jitter_n I) in FP64 with the ladder of
  *         lakde_posterior_factor (info_n = -1 when it fails)
@@ -201,7 +201,8 @@ LAKDE_API int lakde_estep_logrho(int dtype, int64_t N, int64_t D, int64_t npts,
  * P and T [D,D] blocks with batch strides (0 = shared), a, b (in/out), jitter
  * (in/out), nu, logdet_W, mm [N] (mm may be NULL), info [N].  Row n is the
  * kernel centred on point n + kernel_offset of X (a shard's rows; npts >=
- * N + kernel_offset); the per-kernel arrays are indexed by n.
+ * N + kernel_offset); the per-kernel arrays are indexed by n.  A shard's rows are
+ * those of the full launch bit for bit: the order of a row's sums follows npts.
  */
 LAKDE_API int lakde_vi_rows(int dtype, int64_t N, int64_t D, int64_t npts,
                             const void *rowptr, const void *col,
@@ -442,7 +443,9 @@ LAKDE_API int lakde_weighted_gram(int dtype, int64_t N, int64_t D,
  * topk per row block, the point itself excluded at :104-105 unless
  * include_self).  dist [nb, N] (float64, row-major) holds the squared
  * distances of points row0 .. row0 + nb - 1 to all N points of X [N, D]
- * (float64), e.g. |a|^2 + |b|^2 - 2ab from a library GEMM.  Per row: the
+ * (float64), e.g. |a|^2 + |b|^2 - 2ab from a library GEMM, less any constant of
+ * the row; values that are not finite are no distances (index -1 where a row has
+ * fewer than k).  Per row: the
  * k + 8 smallest entries (one pass, a shared-memory candidate buffer with a
  * running threshold) are re-ranked by exact float64 differences, and the k
  * nearest by (exact distance, index) go to out_idx [nb, k] (idx_dtype I32 /

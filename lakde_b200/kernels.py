@@ -243,7 +243,7 @@ def estep_logrho(rowptr, col, X, W_triu, nu, logdet_W, kernel_offset=0, out=None
 
 def vi_rows(rowptr, col, r, X, nu_0, a, b, b_0, jitter, eps, nu, logdet_W, info, logrho, P=None, T=None,
             order=None, mm=None, kernel_offset=0):
-    """Fused per-kernel pass of one VI iteration, one thread per kernel row,
+    """Fused per-kernel pass of one VI iteration, 2 to 32 kernel rows a warp,
     D <= 8 (lakde_vi_rows, see include/lakde_b200.h).  Row n is the kernel
     centred on X[n + kernel_offset] (a shard's rows)."""
     nat.require_cuda(rowptr, col, r, X, a, b, jitter, nu, logdet_W, info, logrho, P, T, order, mm, op="vi_rows")
