@@ -1183,15 +1183,31 @@ __global__ void __launch_bounds__(Cfg<MODE, DP>::THREADS, Cfg<MODE, DP>::CTAS) t
     // the first two tiles have no earlier accumulator to wait for
     if (MODE != MSTEP && grp == 0 && lane < 2) mbar_arrive(conv + lane);
     if (MODE == PRED) {
-      // queries of this warp's lanes with a NaN, which the split would lose
-      const int64_t q0 = (int64_t)(blockIdx.x % g.nqb) * QB + 32 * w4;
+      // this thread's queries with a NaN, which the split would lose: read by the
+      // whole warp, up to 32 dimensions by the thread itself, whose few loads keep
+      // the first tiles waiting less (2,000 kernels x 300 queries at d = 13 37.7 against
+      // 39.4 us; 10,000 x 2,000 at d = 48 1.21 against 1.14 ms)
 #pragma unroll 1
       for (int tl = 0; tl < 2; ++tl) {
-        const int64_t left = g.Nq - (q0 + tl * MT);
+        const int64_t q = (int64_t)(blockIdx.x % g.nqb) * QB + tl * MT + 32 * w4;
+        if constexpr (DP <= 32) {
+          if (q + lane >= g.Nq) break;
+          const float *y = g.Y + (q + lane) * g.ldy;
+          bool nan = false;
 #pragma unroll 4
-        for (int j = 0; j < (left < 32 ? (int)left : 32); ++j)
-          if (K::row_has_nan(g.Y + (q0 + tl * MT + j) * g.ldy, g.D, lane) && lane == j) qnan |= 1u << tl;
+          for (int k = 0; k < g.D / 4; ++k) {
+            const float4 v = reinterpret_cast<const float4 *>(y)[k];
+            nan = nan || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+          }
+          for (int d = g.D & ~3; d < g.D; ++d) nan = nan || y[d] != y[d];
+          if (nan) qnan |= 1u << tl;
+        } else {
+#pragma unroll 4
+          for (int j = 0; j < (g.Nq - q < 32 ? (int)(g.Nq - q) : 32); ++j)
+            if (K::row_has_nan(g.Y + (q + j) * g.ldy, g.D, lane) && lane == j) qnan |= 1u << tl;
+        }
       }
+      __syncwarp();
     }
     for (int t = 0;; ++t) {
       ok = __all_sync(0xffffffffu, ready(t));
